@@ -26,6 +26,7 @@ struct eup_handle {
     void* lat[2] = {nullptr, nullptr};
     void* ghost = nullptr;
     void* xface = nullptr;        // x = 1 / x = l columns, [2][18][m*n] arithmetic type
+    HaloEdgesDevice edges;        // stores of the halo's edge lines (edges.e owned by the handle)
     int64_t* d_itime = nullptr;   // device copy of the step counter (series slot of the drag)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one time step, source lattice 0 or 1
     int cur = 0;
@@ -41,7 +42,6 @@ struct eup_handle {
     int64_t cap = 0;
     double* dscratch = nullptr;  // 64 doubles
     unsigned int* d_bad = nullptr;  // upload check: bit q set when population q had a non-finite value
-    unsigned int* bc_bar = nullptr; // grid barrier of the single-launch halo kernel: arrivals, generation, timeouts
     void* staging = nullptr;
     size_t staging_bytes = 0;
     // state transfers: a second staging buffer and a copy stream, so that the host copy of
@@ -54,7 +54,9 @@ struct eup_handle {
     int64_t itime = 0, series_first = 0;
     bool has_state = false;
     double scale = 1.0;
-    int variant = 0;  // EUP_STEP_VARIANT: bit 0/2 16/8-byte vector stream-collide, bit 1 no CUDA graphs
+    // EUP_STEP_VARIANT: bit 0/2 16/8-byte vector stream-collide, bit 1 no CUDA graphs, bit 12 (set
+    // by default) one launch for all halo blocks; the other bits in launch_stream_collide
+    int variant = 4096;
     bool pbb = false;             // partial-bounce-back model active (solid fraction set)
     void* ns = nullptr;           // solid fraction n_s per interior node, arithmetic type
     int32_t* ns_list = nullptr;   // interior linear indices with n_s > 0, ascending
@@ -139,9 +141,8 @@ Phys<R> make_phys(const eup_handle* h) {
 
 Mask make_mask(const eup_handle* h) { return Mask{h->bits, h->wpr}; }
 
-// The halo kernels' grid barrier when they run as one cooperative launch (EUP_STEP_VARIANT
-// bit 12; measured slower than one launch per block, the default), else none.
-unsigned int* bc_bar(const eup_handle* h) { return (h->variant & 4096) ? h->bc_bar : nullptr; }
+// EUP_STEP_VARIANT without bit 12: one launch per halo block instead of one for all.
+bool bc_separate(const eup_handle* h) { return !(h->variant & 4096); }
 Reduce make_reduce(const eup_handle* h) { return Reduce{h->partials, h->counter, kReduceMaxBlocks}; }
 
 template <typename S, typename R>
@@ -171,7 +172,7 @@ int enqueue_one_step(eup_handle* h, int src_idx, PhaseEvents* pe, size_t s) {
     if (pe) pe->mark(4 * s + 0, h->stream);
     if (h->pbb) {  // partial bounce-back: halo planes, stream-collide, mixing and force of the step
         if (pe) pe->mark(4 * s + 1, h->stream);
-        n += launch_bc<S, R>(src, h->g, bc, ph, h->stream, bc_bar(h));
+        n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h));
         if (pe) pe->mark(4 * s + 2, h->stream);
         launch_pbb_step<S, R>(src, dst, h->g, ph, static_cast<const R*>(h->ns), h->ns_list, h->ns_count,
                               make_reduce(h), h->series, h->cap, h->d_itime, h->stream);
@@ -183,7 +184,7 @@ int enqueue_one_step(eup_handle* h, int src_idx, PhaseEvents* pe, size_t s) {
                              h->cap, h->d_itime, true, h->stream);
     n += 1;
     if (pe) pe->mark(4 * s + 1, h->stream);
-    n += launch_bc<S, R>(src, h->g, bc, ph, h->stream, bc_bar(h));
+    n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h));
     if (pe) pe->mark(4 * s + 2, h->stream);
     // propagation + collision (CODE/SRC/bgk3d.F90:133-138)
     launch_stream_collide<S, R>(src, dst, h->g, ph, h->variant, h->stream);
@@ -205,7 +206,7 @@ void enqueue_boundaries(eup_handle* h) {
     const Lat<S, R> src = make_lat<S, R>(h, h->cur);
     launch_bounce_drag<S, R>(src, h->g, bc, h->blist, h->blinks, h->nblist, true, make_reduce(h), h->series,
                              h->cap, h->d_itime, true, h->stream);
-    h->launches += 1 + launch_bc<S, R>(src, h->g, bc, ph, h->stream, bc_bar(h));
+    h->launches += 1 + launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h));
     if (const int xs = exchange_sides(h)) {  // the plane messages' halo rows, after the halo kernels
         launch_pack_x_rim<S, R>(src, h->g, xs, h->stream);
         h->launches += 1;
@@ -469,14 +470,6 @@ int check_kernel_waits(eup_handle* h, const char* who) {
                     std::string(who) + ": " + std::to_string(n) +
                         " bulk copies of the staged stream-collide kernel did not complete within 2 s; "
                         "the steps since are incomplete");
-    unsigned int bar[3] = {0, 0, 0};
-    CK(h, cudaMemcpy(bar, h->bc_bar, sizeof(bar), cudaMemcpyDeviceToHost));
-    if (bar[2] != 0) {
-        cudaMemset(h->bc_bar, 0, sizeof(bar));  // a barrier that gave up leaves its counter behind
-        return fail(h, EUP_ERR_CUDA,
-                    std::string(who) + ": " + std::to_string(bar[2]) +
-                        " grid-barrier waits of the halo kernel gave up after 1 s; the steps since are incomplete");
-    }
     return EUP_OK;
 }
 
@@ -574,16 +567,19 @@ int eup_create(const eup_config* cfg, eup_handle** out) {
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(scratch)"));
     if ((e = cudaMalloc(&h->d_bad, sizeof(unsigned int))) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(upload check)"));
-    if ((e = cudaMalloc(&h->bc_bar, 3 * sizeof(unsigned int))) != cudaSuccess)
-        return cleanup_fail(cuda_fail(h, e, "cudaMalloc(halo barrier)"));
-    if ((e = cudaMemset(h->bc_bar, 0, 3 * sizeof(unsigned int))) != cudaSuccess)
-        return cleanup_fail(cuda_fail(h, e, "cudaMemset(halo barrier)"));
-    if ((h->variant & 4096) && (e = prepare_bc_fused(h->bc_bar)) != cudaSuccess)
-        return cleanup_fail(cuda_fail(h, e, "halo kernel set-up"));
     const size_t xface_bytes = (size_t)xface_elems(h->g) * h->rbytes;
     if ((e = cudaMalloc(&h->xface, xface_bytes)) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(x-face copy)"));
     cudaMemsetAsync(h->xface, 0, xface_bytes, h->stream);
+    const HaloEdges edges = build_halo_edges(h->g, cfg->bc);
+    HaloEdge* d_edges = nullptr;
+    if ((e = cudaMalloc(&d_edges, sizeof(HaloEdge) * (edges.e.size() + 1))) != cudaSuccess)
+        return cleanup_fail(cuda_fail(h, e, "cudaMalloc(halo edges)"));
+    h->edges.e = d_edges;
+    for (int b = 0; b < 9; ++b) h->edges.first[b] = edges.first[b];
+    if ((e = cudaMemcpyAsync(d_edges, edges.e.data(), sizeof(HaloEdge) * edges.e.size(), cudaMemcpyHostToDevice,
+                             h->stream)) != cudaSuccess)
+        return cleanup_fail(cuda_fail(h, e, "halo edges"));
     if ((e = cudaMalloc(&h->d_itime, sizeof(int64_t))) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(step counter)"));
     cudaMemsetAsync(h->d_itime, 0, sizeof(int64_t), h->stream);
@@ -600,7 +596,7 @@ int eup_destroy(eup_handle* h) {
     drop_graphs(h);
     void* ptrs[] = {h->lat[0], h->lat[1], h->ghost, h->bits, h->blist, h->blinks, h->partials, h->counter,
                     h->series, h->dscratch, h->staging, h->xface, h->d_itime, h->ns, h->d_bad, h->ns_list,
-                    h->bc_bar, h->staging2};
+                    h->staging2, const_cast<HaloEdge*>(h->edges.e)};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (cudaEvent_t e : h->xev)
@@ -1611,7 +1607,7 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
             CK(h, cudaGraphLaunch(h->graph[h->cur], st));
         } else {
             const Lat<S, R> src = make_lat<S, R>(h, h->cur), dst = make_lat<S, R>(h, h->cur ^ 1);
-            launch_bc<S, R>(src, g, bc, ph, st, bc_bar(h));
+            launch_bc<S, R>(src, g, bc, ph, h->edges, st, bc_separate(h));
             launch_pbb_step<S, R>(src, dst, g, ph, ns, h->ns_list, h->ns_count, red, h->series, h->cap, h->d_itime,
                                   st);
         }
@@ -1645,7 +1641,7 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
                     const Lat<S, R> src = buf_lat(cur), dst = buf_lat(next);
                     const uint64_t key = ((uint64_t)1 << 60) | ((uint64_t)cur << 24) | (uint64_t)next;
                     const cudaError_t e_run = step(key, [&] {
-                        launch_bc<S, R>(src, g, bc, ph, st, bc_bar(h));
+                        launch_bc<S, R>(src, g, bc, ph, h->edges, st, bc_separate(h));
                         launch_pbb_step<S, R>(src, dst, g, ph, ns, h->ns_list, h->ns_count, red, nullptr, 0, nullptr,
                                               st);
                     });
@@ -1677,7 +1673,7 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
                                      (uint64_t)in_window;
                 const cudaError_t e_run = step(key, [&] {
                     if (serial) {
-                        launch_bc<S, R>(f, g, bc, ph, st, bc_bar(h));  // the halo of step t, from state t-1
+                        launch_bc<S, R>(f, g, bc, ph, h->edges, st, bc_separate(h));  // the halo of step t, from state t-1
                         launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, st, kAdjAll);
                         return;
                     }
@@ -1686,7 +1682,7 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
                     // nodes run on the side stream beside them; the halo transposes after both
                     cudaEventRecord(side.fork, st);
                     cudaStreamWaitEvent(side.s, side.fork, 0);
-                    launch_bc<S, R>(f, g, bc, ph, side.s, bc_bar(h));
+                    launch_bc<S, R>(f, g, bc, ph, h->edges, side.s, bc_separate(h));
                     launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, side.s, kAdjFaces);
                     cudaEventRecord(side.join, side.s);
                     launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, st, kAdjInterior);

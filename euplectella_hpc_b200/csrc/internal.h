@@ -96,17 +96,52 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[W], const Reduce&
     }
 }
 
-// Halo-plane operations of CODE/SRC/bcond.bc.F90 in the reference's order; returns the
-// number of kernels launched.  With `bar` (three zeroed words of device memory owned by the
-// caller, used by one stream at a time) and a device where prepare_bc_fused found cooperative
-// launches usable in CUDA graphs, all blocks run as phases of one launch separated by grid
-// barriers (measured slower); otherwise, and by default, one launch per block.
+// ---- halo planes (halo.h, halo_plan.cu) -----------------------------------------------
+// One store to an edge line: ghost[dst] = a value of kind.
+enum : int32_t {
+    kEdgeCopy,       // population q of interior node src
+    kEdgeCopyPlus,   //   ... plus the lid's force
+    kEdgeCopyMinus,  //   ... minus it
+    kEdgeOld,        // ghost[src], a halo value no item of a step writes
+    kEdgeOutflow,    // outflow population 10 + q of row src = (j-1) + (k-1) m
+    kEdgeConst       // inflow population 1 + q
+};
+struct HaloEdge {
+    int64_t dst, src;
+    int32_t q, kind;
+};
+// The edge stores of a step, grouped by the block that makes them.
+struct HaloEdges {
+    std::vector<HaloEdge> e;
+    int64_t first[9];
+};
+struct HaloEdgesDevice {
+    const HaloEdge* e = nullptr;
+    int64_t first[9] = {};
+};
+HaloEdges build_halo_edges(const Geo& g, const int bc[6]);
+
+// One face of the halo away from the edge lines: nodes (a, b) of the face, a = 0 .. na-1 and
+// b = 0 .. nb-1, a fastest.  Population t of the five goes to ghost[dst[t] + a + b dst_b] where
+// (a + da, b + db) is on the face (a no-slip block stores one node along a tangential axis;
+// beyond the face lies an edge line).
+enum : int { kFaceNone = -1, kFaceCopy, kFaceCopyX, kFaceOutflow, kFaceConst };
+struct HaloFace {
+    int kind;  // copy from the lattice, from the x-face copy, outflow equilibrium, inflow constants
+    int na, nb;
+    int64_t src_b, dst_b;
+    int q[5], src_q[5], da[5], db[5], lid[5];
+    int64_t src[5], dst[5];
+    int pass;          // >= 0: on row b = nb-1 the old value of population `pass` goes to pass_dst + a first
+    int64_t pass_dst;
+};
+HaloFace record_halo_face(const Geo& g, const int bc[6], int block);
+
+// Halo planes of one step (CODE/SRC/bcond.bc.F90) in one launch, or one launch per block of
+// the reference; returns the number of kernels launched.
 template <typename S, typename R>
-int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, cudaStream_t st,
-              unsigned int* bar = nullptr);
-// Once per device (outside graph capture): occupancy of the single-launch halo kernel, and a
-// cooperative launch captured into a graph and run once, using `bar` (left zeroed).
-cudaError_t prepare_bc_fused(unsigned int* bar);
+int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, const HaloEdgesDevice& edges,
+              cudaStream_t st, bool separate = false);
 
 // Bounce-back on solid voxels touching fluid/halo (CODE/SRC/bcond.obs.F90) and the
 // FP64 momentum-exchange force of the state it reads, written to

@@ -4,297 +4,124 @@
 // (CODE/SRC/probe_global.F90) and the host-layout scatter/gather used by
 // upload and download.  All of it is O(surface) or O(solid surface) work.
 #include "init_eq.h"
-#include <algorithm>
-#include <type_traits>
-
+#include "halo.h"
 #include "internal.h"
 
 namespace eup {
 
 namespace {
 
-// One thread per (a, b) pair of a face loop; a runs fastest.
-struct Range2 {
-    int a0, na, b0, nb;
-    // element `t` of the loop (false beyond its end)
-    __device__ __forceinline__ bool at(int64_t t, int& a, int& b) const {
-        if (t >= (int64_t)na * nb) return false;
-        a = a0 + (int)(t % na);
-        b = b0 + (int)(t / na);
-        return true;
-    }
-    int64_t size() const { return (int64_t)na * nb; }
-    unsigned blocks(int tpb) const {
-        const int64_t t = (int64_t)na * nb;
-        return (unsigned)((t + tpb - 1) / tpb);
-    }
-};
-
 constexpr int kTpb = 256;
 
-// Loads inside the halo kernels go through bc_load: interior nodes of the
-// x = 1 and x = l columns come from the compact x-face copy written by the
-// stream-collide kernel (coalesced in j), other interior nodes from the
-// lattice, halo nodes from the shell.  Every kernel issues all of a thread's
-// loads before its first store (stores to the shell may alias the loads).
-#define LD(q1, i, j, k) bc_load(L, g, (q1) - 1, (i), (j), (k))
-#define ST(q1, i, j, k, v) ghost_store(L, g, (q1) - 1, (i), (j), (k), (v))
+// ---- halo planes ---------------------------------------------------------------------
+//
+// One launch for the halo of a step.  A segment is a run of thread blocks with one job: a face
+// (one thread per node of the face, five populations each) or the edge stores of one of the
+// reference's blocks (one thread per store).  The x faces read the compact x-face copy written
+// by the stream-collide kernel (coalesced in j; a strided read of a column costs a sector per
+// node), the others the lattice.
+//
+// What bounds it on all but the largest lattices is the latency of a short kernel, and there
+// instruction fetch: a launch starts with cold instruction caches, and ncu puts 80 % of the
+// stalls of such kernels on missing instructions.  So the code is kept short and straight: the
+// five copies of every face flag are one piece of code with strides from the plan, and whatever
+// is irregular is in the table instead of in branches.  Halo planes of one step (CUDA events,
+// launch included), as eight dependent launches / as one: 38 / 6.9 us at 64x32x8, 41 / 8.4 us at
+// 256x128x64, 48 / 10.6 us at 384x192x192, 61 / 19.4 us at 768x384x384 FP32.  (One launch with
+// the items' conditions written out: 12 and 23 us at the first two.)
+constexpr int kHaloSegments = 2 * kHaloBlocks;
 
-// ---- front wall, x = l+1 -----------------------------------------------------
 template <typename S, typename R>
-__device__ __forceinline__ void front_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int flag, int64_t tid) {
-    int j, k;
-    if (!r.at(tid, j, k)) return;
-    const int l = g.l, l1 = g.l + 1, m = g.m;
-    if (flag == 0) {  // periodic, CODE/SRC/bcond.bc.F90:75-105 (SERIAL corner line :90)
-        if (j == 0) { const R v = LD(12, 1, m, k); ST(12, l1, 0, k, v); return; }
-        R v[5];
+struct HaloSegment {
+    int kind;  // kFace*, or kSegEdges
+    unsigned count;
+    unsigned na, nb;
+    int64_t src_b, dst_b;
+    const void* src[5];
+    R* dst[5];
+    R w[5];    // 16-bit storage: weight of the population; kFaceConst: the value
+    R add[5];  // what the lid adds
+    int da[5], db[5];
+    int lid, pass;
+    R* pass_dst;
+    const HaloEdge* edges;
+};
+constexpr int kSegEdges = 100;
+
+template <typename S, typename R>
+struct HaloPlan {
+    Lat<S, R> L;
+    Geo g;
+    R force;
+    R inflow[5];
+    unsigned first[kHaloSegments + 1];  // first thread block of each segment
+    HaloSegment<S, R> seg[kHaloSegments];
+};
+
+template <typename S, typename R>
+__device__ __forceinline__ void outflow_row(const Lat<S, R>& L, const Geo& g, int64_t row, R (&v)[5]) {
+    R x[18];
+    const R* col = L.xface + (g.xs + g.xr + row);  // column x = l
 #pragma unroll
-        for (int q = 10; q <= 14; ++q) v[q - 10] = LD(q, 1, j, k);
-#pragma unroll
-        for (int q = 10; q <= 14; ++q) ST(q, l1, j, k, v[q - 10]);
-    } else if (flag == 1) {  // no-slip, :108-124
-        const R v1 = LD(1, l, j, k), v2 = LD(2, l, j, k), v3 = LD(3, l, j, k), v4 = LD(4, l, j, k), v5 = LD(5, l, j, k);
-        ST(12, l1, j - 1, k, v1);
-        ST(13, l1, j, k - 1, v2);
-        ST(10, l1, j + 1, k, v3);
-        ST(11, l1, j, k + 1, v4);
-        ST(14, l1, j, k, v5);
-    } else {  // outflow, :127-169: equilibrium at rho=1 with the (un-normalised) momentum of x=l
-        R a[18];
-#pragma unroll
-        for (int q = 0; q < 18; ++q) a[q] = bc_load(L, g, q, l, j, k);
-        const R xj = a[0] + a[1] + a[2] + a[3] + a[4] - a[9] - a[10] - a[11] - a[12] - a[13];
-        const R yj = a[2] + a[6] + a[7] + a[8] + a[11] - a[0] - a[9] - a[15] - a[16] - a[17];
-        const R zj = a[3] + a[5] + a[6] + a[12] + a[17] - a[1] - a[8] - a[10] - a[14] - a[15];
-        const R rf = R(3), qf = R(1.5), t3 = R(3), one = R(1);
-        const R cvsq = xj * xj + yj * yj + zj * zj;
-        const R cx10 = rf * (-xj - yj) + qf * (t3 * (xj + yj) * (xj + yj) - cvsq);
-        const R cx11 = rf * (-xj - zj) + qf * (t3 * (xj + zj) * (xj + zj) - cvsq);
-        const R cx12 = rf * (-xj + yj) + qf * (t3 * (xj - yj) * (xj - yj) - cvsq);
-        const R cx13 = rf * (-xj + zj) + qf * (t3 * (xj - zj) * (xj - zj) - cvsq);
-        const R cx14 = rf * (-xj) + qf * (t3 * (xj) * (xj) - cvsq);
-        const R p1 = Const<R>::p1(), p2 = Const<R>::p2();
-        ST(10, l1, j, k, p2 * (one + cx10));
-        ST(11, l1, j, k, p2 * (one + cx11));
-        ST(12, l1, j, k, p2 * (one + cx12));
-        ST(13, l1, j, k, p2 * (one + cx13));
-        ST(14, l1, j, k, p1 * (one + cx14));
-    }
+    for (int q = 0; q < 18; ++q) x[q] = col[xface_slot(q) * g.mn];
+    halo_outflow(x, v);
 }
 
-// Outflow border fix, CODE/SRC/bcond.bc.F90:172-203: copies of the edge rows.
 template <typename S, typename R>
-__device__ __forceinline__ void front_fix_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int64_t tid) {
-    int t, side;
-    if (!r.at(tid, t, side)) return;
-    const int l1 = g.l + 1, m = g.m, n = g.n;
-    R lo[5], hi[5];
-    if (side == 0 && t >= 1 && t <= m) {
+__global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<S, R> p) {
+    int s = 0;
 #pragma unroll
-        for (int q = 10; q <= 14; ++q) { lo[q - 10] = LD(q, l1, t, 1); hi[q - 10] = LD(q, l1, t, n); }
+    for (int i = 1; i < kHaloSegments; ++i) s += blockIdx.x >= p.first[i];
+    const HaloSegment<S, R>& f = p.seg[s];
+    const unsigned t = (blockIdx.x - p.first[s]) * kTpb + threadIdx.x;
+    if (t >= f.count) return;
+    R v[5];
+    if (f.kind == kSegEdges) {
+        const HaloEdge e = f.edges[t];
+        if (e.kind <= kEdgeCopyMinus) {
+            v[0] = Store<S, R>::load(p.L.pop[e.q][e.src], e.q, p.L.inv_scale);
+            if (e.kind == kEdgeCopyPlus) v[0] = v[0] + p.force;
+            if (e.kind == kEdgeCopyMinus) v[0] = v[0] - p.force;
+        } else if (e.kind == kEdgeOld) {
+            v[0] = p.L.ghost[e.src];
+        } else if (e.kind == kEdgeConst) {
+            v[0] = p.inflow[e.q];
+        } else {
+            outflow_row(p.L, p.g, e.src, v);
+            v[0] = e.q == 0 ? v[0] : (e.q == 1 ? v[1] : (e.q == 2 ? v[2] : (e.q == 3 ? v[3] : v[4])));
+        }
+        p.L.ghost[e.dst] = v[0];
+        return;
+    }
+    const unsigned b = t / f.na, a = t - b * f.na;
+    const int64_t from = a + b * f.src_b, to = a + b * f.dst_b;
+    if (f.kind == kFaceOutflow) {
+        outflow_row(p.L, p.g, from, v);
+    } else if (f.kind == kFaceConst) {
 #pragma unroll
-        for (int q = 10; q <= 14; ++q) { ST(q, l1, t, 0, lo[q - 10]); ST(q, l1, t, n + 1, hi[q - 10]); }
-    }
-    if (side == 1 && t >= 1 && t <= n) {
+        for (int c = 0; c < 5; ++c) v[c] = f.w[c];
+    } else if (!DevStore<S>::value || f.kind == kFaceCopyX) {
 #pragma unroll
-        for (int q = 10; q <= 14; ++q) { lo[q - 10] = LD(q, l1, 1, t); hi[q - 10] = LD(q, l1, m, t); }
+        for (int c = 0; c < 5; ++c) v[c] = static_cast<const R*>(f.src[c])[from];
+    } else {
+        if constexpr (DevStore<S>::value) {
+            S raw[5];
 #pragma unroll
-        for (int q = 10; q <= 14; ++q) { ST(q, l1, 0, t, lo[q - 10]); ST(q, l1, m + 1, t, hi[q - 10]); }
-    }
-}
-
-// ---- rear wall, x = 0 ----------------------------------------------------------
-template <typename S, typename R>
-__device__ __forceinline__ void rear_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int flag, R u_inflow, int64_t tid) {
-    int j, k;
-    if (!r.at(tid, j, k)) return;
-    const int l = g.l, m1 = g.m + 1;
-    if (flag == 0) {  // periodic, :210-238 (SERIAL corner line :223)
-        if (j == 0) { const R v = LD(1, l, 1, k); ST(1, 0, m1, k, v); return; }
-        R v[5];
+            for (int c = 0; c < 5; ++c) raw[c] = static_cast<const S*>(f.src[c])[from];
 #pragma unroll
-        for (int q = 1; q <= 5; ++q) v[q - 1] = LD(q, l, j, k);
+            for (int c = 0; c < 5; ++c) v[c] = f.w[c] + DevStore<S>::to_f(raw[c]) * p.L.inv_scale;
+        }
+    }
+    if (f.lid) {  // a moving lid: populations 2 and 11 alone
 #pragma unroll
-        for (int q = 1; q <= 5; ++q) ST(q, 0, j, k, v[q - 1]);
-    } else if (flag == 1) {  // no-slip, :241-257
-        const R v10 = LD(10, 1, j, k), v11 = LD(11, 1, j, k), v12 = LD(12, 1, j, k), v13 = LD(13, 1, j, k),
-                v14 = LD(14, 1, j, k);
-        ST(3, 0, j - 1, k, v10);
-        ST(4, 0, j, k - 1, v11);
-        ST(1, 0, j + 1, k, v12);
-        ST(2, 0, j, k + 1, v13);
-        ST(5, 0, j, k, v14);
-    } else {  // inflow, uniform, :260-321
-        const R xj = u_inflow, yj = R(0), zj = R(0);
-        const R rf = R(3), qf = R(1.5), t3 = R(3), one = R(1);
-        const R cvsq = xj * xj + yj * yj + zj * zj;
-        const R cx01 = rf * (xj - yj) + qf * (t3 * (xj - yj) * (xj - yj) - cvsq);
-        const R cx02 = rf * (xj - zj) + qf * (t3 * (xj - zj) * (xj - zj) - cvsq);
-        const R cx03 = rf * (xj + yj) + qf * (t3 * (xj + yj) * (xj + yj) - cvsq);
-        const R cx04 = rf * (xj + zj) + qf * (t3 * (xj + zj) * (xj + zj) - cvsq);
-        const R cx05 = rf * (xj) + qf * (t3 * (xj) * (xj) - cvsq);
-        const R p1 = Const<R>::p1(), p2 = Const<R>::p2();
-        ST(1, 0, j, k, p2 * (one + cx01));
-        ST(2, 0, j, k, p2 * (one + cx02));
-        ST(3, 0, j, k, p2 * (one + cx03));
-        ST(4, 0, j, k, p2 * (one + cx04));
-        ST(5, 0, j, k, p1 * (one + cx05));
+        for (int c = 0; c < 5; ++c)
+            if (f.lid & (1 << c)) v[c] = v[c] + f.add[c];
     }
+    if (f.pass >= 0 && b == f.nb - 1) f.pass_dst[a] = f.dst[f.pass][to];
+#pragma unroll
+    for (int c = 0; c < 5; ++c)
+        if (a + f.da[c] < f.na && b + f.db[c] < f.nb) f.dst[c][to] = v[c];
 }
-
-// ---- up wall, z = n+1 -------------------------------------------------------------
-template <typename S, typename R>
-__device__ __forceinline__ void up_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int flag, R force, int64_t tid) {
-    int i, j;
-    if (!r.at(tid, i, j)) return;
-    const int n = g.n, n1 = g.n + 1;
-    if (flag == 0) {  // periodic, :385-409
-        const R v2 = LD(2, i, j, 1), v9 = LD(9, i, j, 1), v11 = LD(11, i, j, 1), v15 = LD(15, i, j, 1),
-                v16 = LD(16, i, j, 1);
-        ST(2, i, j, n1, v2);
-        ST(9, i, j, n1, v9);
-        ST(11, i, j, n1, v11);
-        ST(15, i, j, n1, v15);
-        ST(16, i, j, n1, v16);
-    } else if (flag == 1 || flag == 2) {  // no-slip :412-428, lid :431-447
-        const R v6 = LD(6, i, j, n), v13 = LD(13, i, j, n), v18 = LD(18, i, j, n), v4 = LD(4, i, j, n),
-                v7 = LD(7, i, j, n);
-        ST(15, i, j, n1, v6);
-        ST(2, i - 1, j, n1, flag == 2 ? v13 + force : v13);
-        ST(9, i, j - 1, n1, v18);
-        ST(11, i + 1, j, n1, flag == 2 ? v4 - force : v4);
-        ST(16, i, j + 1, n1, v7);
-    } else {  // free-slip over i = 0..l+1, j = 0..m+1, :450-468
-        const R v6 = LD(6, i, j, n), v13 = LD(13, i, j, n), v18 = LD(18, i, j, n), v4 = LD(4, i, j, n),
-                v7 = LD(7, i, j, n);
-        ST(15, i, j, n1, v6);
-        ST(11, i, j, n1, v13);
-        ST(16, i, j, n1, v18);
-        ST(2, i, j, n1, v4);
-        ST(9, i, j, n1, v7);
-    }
-}
-
-// ---- down wall, z = 0 ---------------------------------------------------------------
-template <typename S, typename R>
-__device__ __forceinline__ void down_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int flag, int64_t tid) {
-    int i, j;
-    if (!r.at(tid, i, j)) return;
-    const int n = g.n;
-    if (flag == 0) {  // periodic, :472-496
-        const R v4 = LD(4, i, j, n), v6 = LD(6, i, j, n), v7 = LD(7, i, j, n), v13 = LD(13, i, j, n),
-                v18 = LD(18, i, j, n);
-        ST(4, i, j, 0, v4);
-        ST(6, i, j, 0, v6);
-        ST(7, i, j, 0, v7);
-        ST(13, i, j, 0, v13);
-        ST(18, i, j, 0, v18);
-    } else if (flag == 1) {  // no-slip, :499-515
-        const R v15 = LD(15, i, j, 1), v11 = LD(11, i, j, 1), v16 = LD(16, i, j, 1), v2 = LD(2, i, j, 1),
-                v9 = LD(9, i, j, 1);
-        ST(6, i, j, 0, v15);
-        ST(4, i - 1, j, 0, v11);
-        ST(7, i, j - 1, 0, v16);
-        ST(13, i + 1, j, 0, v2);
-        ST(18, i, j + 1, 0, v9);
-    } else {  // free-slip, :518-530
-        const R v15 = LD(15, i, j, 1), v11 = LD(11, i, j, 1), v16 = LD(16, i, j, 1), v2 = LD(2, i, j, 1),
-                v9 = LD(9, i, j, 1);
-        ST(6, i, j, 0, v15);
-        ST(13, i, j, 0, v11);
-        ST(18, i, j, 0, v16);
-        ST(4, i, j, 0, v2);
-        ST(7, i, j, 0, v9);
-    }
-}
-
-// ---- left wall, y = 0 ------------------------------------------------------------------
-template <typename S, typename R>
-__device__ __forceinline__ void left_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int flag, int64_t tid) {
-    int i, k;
-    if (!r.at(tid, i, k)) return;
-    const int l = g.l, m = g.m;
-    if (flag == 0) {  // periodic, :535-560 (corner line :547)
-        if (i == 0) { const R v = LD(3, l, m, k); ST(3, 0, 0, k, v); return; }
-        const R v3 = LD(3, i, m, k), v7 = LD(7, i, m, k), v8 = LD(8, i, m, k), v9 = LD(9, i, m, k),
-                v12 = LD(12, i, m, k);
-        ST(3, i, 0, k, v3);
-        ST(7, i, 0, k, v7);
-        ST(8, i, 0, k, v8);
-        ST(9, i, 0, k, v9);
-        ST(12, i, 0, k, v12);
-    } else if (flag == 1) {  // no-slip, :563-579
-        const R v17 = LD(17, i, 1, k), v1 = LD(1, i, 1, k), v10 = LD(10, i, 1, k), v16 = LD(16, i, 1, k),
-                v18 = LD(18, i, 1, k);
-        ST(8, i, 0, k, v17);
-        ST(12, i + 1, 0, k, v1);
-        ST(3, i - 1, 0, k, v10);
-        ST(7, i, 0, k - 1, v16);
-        ST(9, i, 0, k + 1, v18);
-    } else {  // free-slip, :582-594
-        const R v17 = LD(17, i, 1, k), v1 = LD(1, i, 1, k), v10 = LD(10, i, 1, k), v16 = LD(16, i, 1, k),
-                v18 = LD(18, i, 1, k);
-        ST(8, i, 0, k, v17);
-        ST(3, i, 0, k, v1);
-        ST(12, i, 0, k, v10);
-        ST(9, i, 0, k, v16);
-        ST(7, i, 0, k, v18);
-    }
-}
-
-// ---- right wall, y = m+1 ------------------------------------------------------------------
-template <typename S, typename R>
-__device__ __forceinline__ void right_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int flag, int64_t tid) {
-    int i, k;
-    if (!r.at(tid, i, k)) return;
-    const int m = g.m, m1 = g.m + 1, l1 = g.l + 1;
-    if (flag == 0) {  // periodic, :600-625 (corner line :612)
-        if (i == 0) { const R v = LD(10, 1, 1, k); ST(10, l1, m1, k, v); return; }
-        const R v1 = LD(1, i, 1, k), v10 = LD(10, i, 1, k), v16 = LD(16, i, 1, k), v17 = LD(17, i, 1, k),
-                v18 = LD(18, i, 1, k);
-        ST(1, i, m1, k, v1);
-        ST(10, i, m1, k, v10);
-        ST(16, i, m1, k, v16);
-        ST(17, i, m1, k, v17);
-        ST(18, i, m1, k, v18);
-    } else if (flag == 1) {  // no-slip, :628-644
-        const R v3 = LD(3, i, m, k), v7 = LD(7, i, m, k), v8 = LD(8, i, m, k), v9 = LD(9, i, m, k),
-                v12 = LD(12, i, m, k);
-        ST(10, i + 1, m1, k, v3);
-        ST(16, i, m1, k + 1, v7);
-        ST(17, i, m1, k, v8);
-        ST(18, i, m1, k - 1, v9);
-        ST(1, i - 1, m1, k, v12);
-    } else {  // free-slip, :647-659
-        const R v3 = LD(3, i, m, k), v7 = LD(7, i, m, k), v8 = LD(8, i, m, k), v9 = LD(9, i, m, k),
-                v12 = LD(12, i, m, k);
-        ST(1, i, m1, k, v3);
-        ST(18, i, m1, k, v7);
-        ST(17, i, m1, k, v8);
-        ST(16, i, m1, k, v9);
-        ST(10, i, m1, k, v12);
-    }
-}
-
-// Free-slip edge fixes, CODE/SRC/bcond.bc.F90:663-690.
-template <typename S, typename R>
-__device__ __forceinline__ void edge_fix_body(const Lat<S, R>& L, const Geo& g, const Range2& r, int fixes, int64_t tid) {
-    int i, dummy;
-    if (!r.at(tid, i, dummy)) return;
-    const int m = g.m, m1 = g.m + 1, n = g.n, n1 = g.n + 1;
-    const R v1 = (fixes & 1) ? LD(18, i, 1, n) : R(0);
-    const R v2 = (fixes & 2) ? LD(7, i, m, n) : R(0);
-    const R v3 = (fixes & 4) ? LD(9, i, m, 1) : R(0);
-    const R v4 = (fixes & 8) ? LD(16, i, 1, 1) : R(0);
-    if (fixes & 1) ST(9, i, 0, n1, v1);
-    if (fixes & 2) ST(16, i, m1, n1, v2);
-    if (fixes & 4) ST(18, i, m1, 0, v3);
-    if (fixes & 8) ST(7, i, 0, 0, v4);
-}
-
-#undef LD
-#undef ST
 
 // ---- bounce-back + momentum exchange ---------------------------------------------------
 //
@@ -308,130 +135,6 @@ __device__ __forceinline__ void edge_fix_body(const Lat<S, R>& L, const Geo& g, 
 // wrapped node and its interior value is used.  The force of the state read
 // goes to series[itime % cap], itime read from device memory; with `advance`
 // the last block then increments the device step counter.
-
-// One kernel per halo block (the reference's blocks as separate launches).
-template <typename S, typename R>
-__global__ void k_front(Lat<S, R> L, Geo g, Range2 r, int flag) {
-    front_body<S, R>(L, g, r, flag, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_front_fix(Lat<S, R> L, Geo g, Range2 r) {
-    front_fix_body<S, R>(L, g, r, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_rear(Lat<S, R> L, Geo g, Range2 r, int flag, R u_inflow) {
-    rear_body<S, R>(L, g, r, flag, u_inflow, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_up(Lat<S, R> L, Geo g, Range2 r, int flag, R force) {
-    up_body<S, R>(L, g, r, flag, force, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_down(Lat<S, R> L, Geo g, Range2 r, int flag) {
-    down_body<S, R>(L, g, r, flag, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_left(Lat<S, R> L, Geo g, Range2 r, int flag) {
-    left_body<S, R>(L, g, r, flag, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_right(Lat<S, R> L, Geo g, Range2 r, int flag) {
-    right_body<S, R>(L, g, r, flag, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-template <typename S, typename R>
-__global__ void k_edge_fix(Lat<S, R> L, Geo g, Range2 r, int fixes) {
-    edge_fix_body<S, R>(L, g, r, fixes, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// ---- all halo blocks in one launch (opt-in: EUP_STEP_VARIANT bit 12) ------------------
-// Measured slower than one launch per block on B200 (768x384x384: 0.100 ms against 0.060 ms
-// of halo planes per step; 192x96x96 as well), kept as a tested alternative.
-// The blocks of one step as phases of a single kernel, in the same order, with a grid-wide
-// barrier between phases where the separate launches had a kernel boundary: every element of
-// a phase sees every store of the phases before it, exactly as with one launch per block, so
-// the results are the same bits.  The grid is launched cooperatively (all CTAs resident); the
-// barrier is this library's own (one arrival counter and one generation word per handle, in
-// device memory), and its wait is bounded: after kBarrierWaitNs it counts a timeout in the
-// barrier's third word, which the host reports, and goes on instead of waiting forever.
-enum : int { kBcFront = 0, kBcFrontFix, kBcRear, kBcUp, kBcDown, kBcLeft, kBcRight, kBcEdgeFix };
-struct BcPhase {
-    int kind, flag;
-    Range2 r;
-};
-template <typename R>
-struct BcPlan {
-    int n;
-    BcPhase ph[8];
-    R u_inflow, force;
-};
-
-constexpr uint64_t kBarrierWaitNs = 1000000000ull;
-
-__device__ __forceinline__ uint64_t bc_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// bar[0] arrivals, bar[1] generation, bar[2] timeouts (zero when the handle is created)
-__device__ __forceinline__ void grid_barrier(unsigned int* bar) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned int* gen = bar + 1;
-        const unsigned int g0 = *gen;
-        __threadfence();
-        const unsigned int arrived = atomicAdd(bar, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            bar[0] = 0u;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            const uint64_t t0 = bc_ns();
-            while (*gen == g0) {
-                if (bc_ns() - t0 > kBarrierWaitNs) {
-                    atomicAdd(bar + 2, 1u);
-                    break;
-                }
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-template <typename S, typename R>
-__global__ void __launch_bounds__(kTpb) k_bc_all(Lat<S, R> L, Geo g, BcPlan<R> plan, unsigned int* bar) {
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t nt = (int64_t)gridDim.x * blockDim.x;
-    for (int p = 0; p < plan.n; ++p) {
-        const BcPhase ph = plan.ph[p];
-        const int64_t work = (int64_t)ph.r.na * ph.r.nb;
-        for (int64_t t = t0; t < work; t += nt) {
-            switch (ph.kind) {
-                case kBcFront: front_body<S, R>(L, g, ph.r, ph.flag, t); break;
-                case kBcFrontFix: front_fix_body<S, R>(L, g, ph.r, t); break;
-                case kBcRear: rear_body<S, R>(L, g, ph.r, ph.flag, plan.u_inflow, t); break;
-                case kBcUp: up_body<S, R>(L, g, ph.r, ph.flag, plan.force, t); break;
-                case kBcDown: down_body<S, R>(L, g, ph.r, ph.flag, t); break;
-                case kBcLeft: left_body<S, R>(L, g, ph.r, ph.flag, t); break;
-                case kBcRight: right_body<S, R>(L, g, ph.r, ph.flag, t); break;
-                default: edge_fix_body<S, R>(L, g, ph.r, ph.flag, t); break;
-            }
-        }
-        if (p + 1 < plan.n) grid_barrier(bar);
-    }
-}
-
-// Co-resident CTAs of k_bc_all per device and storage type (0: not measured / not usable).
-constexpr int kBcMaxDevices = 64;
-int g_bc_fused_blocks[kBcMaxDevices][4] = {};
-bool g_bc_fused_ok[kBcMaxDevices] = {};
-
-template <typename S> constexpr int bc_type_index() {
-    return sizeof(S) == 4 ? 0 : sizeof(S) == 8 ? 1 : std::is_same<S, __half>::value ? 2 : 3;
-}
-
-__global__ void k_coop_probe(unsigned int* bar) { grid_barrier(bar); }
 
 template <typename S, typename R>
 __global__ void k_bounce_drag(Lat<S, R> L, Geo g, int per_x, int per_y, int per_z, const int32_t* list,
@@ -899,104 +602,65 @@ void launch_unpack_x(const Lat<S, R>& L, const Geo& g, int side, const R* in, cu
 }
 
 template <typename S, typename R>
-int launch_bc_fused(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, unsigned int* bar,
-                    cudaStream_t st) {
-    const int l = g.l, m = g.m, n = g.n;
-    BcPlan<R> plan;
-    plan.n = 0;
-    plan.u_inflow = ph.u_inflow;
-    plan.force = ph.force;
-    auto add = [&](int kind, int flag, Range2 r) { plan.ph[plan.n++] = BcPhase{kind, flag, r}; };
-    if (bc[0] != 6) {
-        const int f = bc[0];
-        add(kBcFront, f, (f == 0) ? Range2{0, m + 1, 1, n} : Range2{1, m, 1, n});
-        if (f == 5) add(kBcFrontFix, 0, Range2{0, (m > n ? m : n) + 1, 0, 2});
-    }
-    if (bc[1] != 6) {
-        const int f = bc[1];
-        add(kBcRear, f, (f == 0) ? Range2{0, m + 1, 1, n} : (f == 1) ? Range2{1, m, 1, n} : Range2{0, m + 2, 0, n + 2});
-    }
-    add(kBcUp, bc[4], (bc[4] == 3) ? Range2{0, l + 2, 0, m + 2} : Range2{1, l, 1, m});
-    add(kBcDown, bc[5], Range2{1, l, 1, m});
-    add(kBcLeft, bc[3], (bc[3] == 0) ? Range2{0, l + 1, 1, n} : Range2{1, l, 1, n});
-    add(kBcRight, bc[2], (bc[2] == 0) ? Range2{0, l + 1, 1, n} : Range2{1, l, 1, n});
-    const int fixes = ((bc[3] == 3 && bc[4] == 3) ? 1 : 0) | ((bc[2] == 3 && bc[4] == 3) ? 2 : 0) |
-                      ((bc[2] == 3 && bc[5] == 3) ? 4 : 0) | ((bc[3] == 3 && bc[5] == 3) ? 8 : 0);
-    if (fixes) add(kBcEdgeFix, fixes, Range2{1, l, 0, 1});
-    int64_t need = 1;
-    for (int p = 0; p < plan.n; ++p) need = std::max<int64_t>(need, (plan.ph[p].r.size() + kTpb - 1) / kTpb);
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kBcMaxDevices) return -1;
-    const int cap = g_bc_fused_blocks[dev][bc_type_index<S>()];
-    if (!g_bc_fused_ok[dev] || cap <= 0) return -1;
-    unsigned grid = (unsigned)std::min<int64_t>(need, cap);
-    Lat<S, R> Lc = L;
-    Geo gc = g;
-    void* args[] = {&Lc, &gc, &plan, &bar};
-    if (cudaLaunchCooperativeKernel((const void*)k_bc_all<S, R>, dim3(grid), dim3(kTpb), args, 0, st) != cudaSuccess)
-        return -1;
-    return 1;
-}
-
-template <typename S, typename R>
-int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, cudaStream_t st,
-              unsigned int* bar) {
-    if (bar) {  // one cooperative launch for all blocks when the device allows it
-        const int n = launch_bc_fused<S, R>(L, g, bc, ph, bar, st);
-        if (n > 0) return n;
-        cudaGetLastError();  // a refused cooperative launch leaves nothing behind: use one launch per block
-    }
-    const int l = g.l, m = g.m, n = g.n;
-    int launches = 4;
-    // front (an x-slab exchange face gets its plane from the neighbour instead)
-    if (bc[0] != 6) {
+int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, const HaloEdgesDevice& edges,
+              cudaStream_t st, bool separate) {
+    HaloPlan<S, R> p{};
+    p.L = L;
+    p.g = g;
+    p.force = ph.force;
+    halo_inflow(ph.u_inflow, p.inflow);
+    int n = 0, launches = 0;
+    auto launch = [&] {
+        if (n == 0) return;
+        const unsigned blocks = p.first[n];
+        for (int s = n; s <= kHaloSegments; ++s) p.first[s] = 0xffffffffu;  // no block reaches them
+        k_halo<S, R><<<blocks, kTpb, 0, st>>>(p);
         ++launches;
-        const int f = bc[0];
-        Range2 r = (f == 0) ? Range2{0, m + 1, 1, n} : Range2{1, m, 1, n};
-        k_front<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, f);
-        if (f == 5) {
-            Range2 rf{0, (m > n ? m : n) + 1, 0, 2};
-            k_front_fix<S, R><<<rf.blocks(kTpb), kTpb, 0, st>>>(L, g, rf);
-            ++launches;
+        n = 0;
+    };
+    auto add = [&](const HaloSegment<S, R>& f) {
+        p.seg[n] = f;
+        p.first[n + 1] = p.first[n] + (f.count + kTpb - 1) / kTpb;
+        ++n;
+    };
+    for (int b = 0; b < kHaloBlocks; ++b) {
+        p.first[0] = 0;
+        const HaloFace face = record_halo_face(g, bc, b);
+        if (face.kind != kFaceNone) {
+            HaloSegment<S, R> f{};
+            f.kind = face.kind;
+            f.na = (unsigned)face.na;
+            f.nb = (unsigned)face.nb;
+            f.count = f.na * f.nb;
+            f.src_b = face.src_b;
+            f.dst_b = face.dst_b;
+            f.pass = face.pass;
+            f.pass_dst = L.ghost + face.pass_dst;
+            for (int c = 0; c < 5; ++c) {
+                f.dst[c] = L.ghost + face.dst[c];
+                f.da[c] = face.da[c];
+                f.db[c] = face.db[c];
+                f.add[c] = face.lid[c] < 0 ? -ph.force : ph.force;
+                f.lid |= face.lid[c] != 0 ? 1 << c : 0;
+                if (face.kind == kFaceConst) f.w[c] = p.inflow[face.src_q[c]];
+                if (face.kind == kFaceCopyX) f.src[c] = L.xface + face.src[c];
+                if (face.kind == kFaceCopy) {
+                    f.src[c] = L.pop[face.src_q[c]] + face.src[c];
+                    f.w[c] = wclass_of(face.src_q[c]) == 1 ? R(1.0 / 18.0) : R(1.0 / 36.0);
+                }
+            }
+            add(f);
         }
+        if (edges.first[b + 1] > edges.first[b]) {
+            HaloSegment<S, R> f{};
+            f.kind = kSegEdges;
+            f.count = (unsigned)(edges.first[b + 1] - edges.first[b]);
+            f.edges = edges.e + edges.first[b];
+            add(f);
+        }
+        if (separate) launch();
     }
-    // rear
-    if (bc[1] != 6) {
-        ++launches;
-        const int f = bc[1];
-        Range2 r = (f == 0) ? Range2{0, m + 1, 1, n} : (f == 1) ? Range2{1, m, 1, n} : Range2{0, m + 2, 0, n + 2};
-        k_rear<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, f, ph.u_inflow);
-    }
-    // up
-    {
-        const int f = bc[4];
-        Range2 r = (f == 3) ? Range2{0, l + 2, 0, m + 2} : Range2{1, l, 1, m};
-        k_up<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, f, ph.force);
-    }
-    // down
-    {
-        Range2 r{1, l, 1, m};
-        k_down<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, bc[5]);
-    }
-    // left
-    {
-        const int f = bc[3];
-        Range2 r = (f == 0) ? Range2{0, l + 1, 1, n} : Range2{1, l, 1, n};
-        k_left<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, f);
-    }
-    // right
-    {
-        const int f = bc[2];
-        Range2 r = (f == 0) ? Range2{0, l + 1, 1, n} : Range2{1, l, 1, n};
-        k_right<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, f);
-    }
-    const int fixes = ((bc[3] == 3 && bc[4] == 3) ? 1 : 0) | ((bc[2] == 3 && bc[4] == 3) ? 2 : 0) |
-                      ((bc[2] == 3 && bc[5] == 3) ? 4 : 0) | ((bc[3] == 3 && bc[5] == 3) ? 8 : 0);
-    if (fixes) {
-        Range2 r{1, l, 0, 1};
-        k_edge_fix<S, R><<<r.blocks(kTpb), kTpb, 0, st>>>(L, g, r, fixes);
-        ++launches;
-    }
+    launch();
     return launches;
 }
 
@@ -1079,8 +743,8 @@ void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStre
 }
 
 #define EUP_INST(S, R)                                                                                 \
-    template int launch_bc<S, R>(const Lat<S, R>&, const Geo&, const int*, const Phys<R>&, cudaStream_t,   \
-                                 unsigned int*);                                                          \
+    template int launch_bc<S, R>(const Lat<S, R>&, const Geo&, const int*, const Phys<R>&, const HaloEdgesDevice&, \
+                                 cudaStream_t, bool);                                                     \
     template void launch_bounce_drag<S, R>(const Lat<S, R>&, const Geo&, const int*, const int32_t*,   \
                                            const uint64_t*, int64_t, bool, const Reduce&, double*,     \
                                            int64_t, int64_t*, bool, cudaStream_t);                     \
@@ -1110,46 +774,5 @@ EUP_INST(float, float)
 EUP_INST(double, double)
 EUP_INST(__half, float)
 EUP_INST(__nv_bfloat16, float)
-
-cudaError_t prepare_bc_fused(unsigned int* bar) {
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kBcMaxDevices) return cudaSuccess;  // separate launches there
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    int coop = 0;
-    if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return e;
-    const void* ks[4] = {(const void*)k_bc_all<float, float>, (const void*)k_bc_all<double, double>,
-                         (const void*)k_bc_all<__half, float>, (const void*)k_bc_all<__nv_bfloat16, float>};
-    for (int t = 0; t < 4; ++t) {
-        int per_sm = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ks[t], kTpb, 0)) != cudaSuccess) return e;
-        g_bc_fused_blocks[dev][t] = per_sm * sms;
-    }
-    if (!coop) return cudaSuccess;
-    // a cooperative launch must survive stream capture (every step runs as a CUDA graph):
-    // capture one on a private stream, instantiate and run the graph once
-    cudaStream_t s = nullptr;
-    if ((e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)) != cudaSuccess) return e;
-    bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    void* args[] = {&bar};
-    const bool launched =
-        ok && cudaLaunchCooperativeKernel((const void*)k_coop_probe, dim3(2), dim3(32), args, 0, s) == cudaSuccess;
-    cudaGraph_t graph = nullptr;
-    ok = (cudaStreamEndCapture(s, &graph) == cudaSuccess) && launched && graph;
-    cudaGraphExec_t exec = nullptr;
-    if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-    if (ok) ok = cudaGraphLaunch(exec, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
-    unsigned int word[3] = {1, 0, 1};
-    if (ok) ok = cudaMemcpy(word, bar, sizeof(word), cudaMemcpyDeviceToHost) == cudaSuccess;
-    // the probe's two CTAs met at the barrier: no timeout, arrivals back to zero, one generation
-    ok = ok && word[0] == 0 && word[1] == 1 && word[2] == 0;
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(s);
-    cudaGetLastError();
-    g_bc_fused_ok[dev] = ok;
-    return cudaMemset(bar, 0, 3 * sizeof(unsigned int));
-}
 
 }  // namespace eup
