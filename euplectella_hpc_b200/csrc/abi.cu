@@ -32,9 +32,9 @@ struct eup_handle {
     int cur = 0;
     uint32_t* bits = nullptr;
     int wpr = 0;
-    int32_t* blist = nullptr;
-    uint64_t* blinks = nullptr;   // neighbour classification of each boundary-solid voxel
+    int32_t* blist = nullptr;     // solid voxels touching fluid or halo
     int64_t nblist = 0;
+    LinksDevice links;            // their links (arrays owned by the handle)
     int64_t nsolid = 0;           // solid voxels of the installed mask
     double* partials = nullptr;
     unsigned int* counter = nullptr;
@@ -147,9 +147,8 @@ Reduce make_reduce(const eup_handle* h) { return Reduce{h->partials, h->counter,
 
 template <typename S, typename R>
 void enqueue_drag_only(eup_handle* h) {
-    const int bc[6] = {h->cfg.bc[0], h->cfg.bc[1], h->cfg.bc[2], h->cfg.bc[3], h->cfg.bc[4], h->cfg.bc[5]};
-    launch_bounce_drag<S, R>(make_lat<S, R>(h, h->cur), h->g, bc, h->blist, h->blinks, h->nblist, false,
-                             make_reduce(h), h->series, h->cap, h->d_itime, false, h->stream);
+    launch_force<S, R>(make_lat<S, R>(h, h->cur), h->g, h->links, make_reduce(h), h->series, h->cap, h->d_itime,
+                       h->stream);
 }
 
 // Events bracketing the phases of each step when profiling: ev[4*s + p].
@@ -180,11 +179,11 @@ int enqueue_one_step(eup_handle* h, int src_idx, PhaseEvents* pe, size_t s) {
         return n + 2;
     }
     // boundaries: bounce-back then halo planes (CODE/SRC/boundaries.F90:36-49,235-248)
-    launch_bounce_drag<S, R>(src, h->g, bc, h->blist, h->blinks, h->nblist, true, make_reduce(h), h->series,
-                             h->cap, h->d_itime, true, h->stream);
-    n += 1;
+    const ForceSum force = launch_bounce<S, R>(src, h->g, h->links, make_reduce(h), h->series, h->cap, h->d_itime,
+                                               h->stream);
+    n += force.blocks > 0;
     if (pe) pe->mark(4 * s + 1, h->stream);
-    n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h));
+    n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h), &force);
     if (pe) pe->mark(4 * s + 2, h->stream);
     // propagation + collision (CODE/SRC/bgk3d.F90:133-138)
     launch_stream_collide<S, R>(src, dst, h->g, ph, h->variant, h->stream);
@@ -204,9 +203,9 @@ void enqueue_boundaries(eup_handle* h) {
     const Phys<R> ph = make_phys<R>(h);
     const int bc[6] = {h->cfg.bc[0], h->cfg.bc[1], h->cfg.bc[2], h->cfg.bc[3], h->cfg.bc[4], h->cfg.bc[5]};
     const Lat<S, R> src = make_lat<S, R>(h, h->cur);
-    launch_bounce_drag<S, R>(src, h->g, bc, h->blist, h->blinks, h->nblist, true, make_reduce(h), h->series,
-                             h->cap, h->d_itime, true, h->stream);
-    h->launches += 1 + launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h));
+    const ForceSum force = launch_bounce<S, R>(src, h->g, h->links, make_reduce(h), h->series, h->cap, h->d_itime,
+                                               h->stream);
+    h->launches += (force.blocks > 0) + launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h), &force);
     if (const int xs = exchange_sides(h)) {  // the plane messages' halo rows, after the halo kernels
         launch_pack_x_rim<S, R>(src, h->g, xs, h->stream);
         h->launches += 1;
@@ -594,7 +593,8 @@ int eup_destroy(eup_handle* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->xfer) cudaStreamSynchronize(h->xfer);
     drop_graphs(h);
-    void* ptrs[] = {h->lat[0], h->lat[1], h->ghost, h->bits, h->blist, h->blinks, h->partials, h->counter,
+    void* ptrs[] = {h->lat[0], h->lat[1], h->ghost, h->bits, h->blist, const_cast<FluidLink*>(h->links.fluid),
+                    const_cast<HaloLink*>(h->links.halo), h->partials, h->counter,
                     h->series, h->dscratch, h->staging, h->xface, h->d_itime, h->ns, h->d_bad, h->ns_list,
                     h->staging2, const_cast<HaloEdge*>(h->edges.e)};
     for (void* p : ptrs)
@@ -632,46 +632,59 @@ int check_obstacles(eup_handle* h, const char* who, int64_t nsolid, int64_t on_f
 
 // Installs `bits` (m*n*wpr words, owned by the handle from here on; null or
 // nsolid == 0: no solids) in place of the current mask: the list of boundary
-// solids, their link words, and the drag of the current state.  Every buffer is
-// allocated before the current mask is released, so a failed allocation leaves
-// the handle as it was.
-int install_mask(eup_handle* h, uint32_t* bits, int64_t nsolid) {
+// solids, their links, and the drag of the current state.  Everything is built
+// before the current mask is released, so a failed allocation leaves the handle
+// as it was.
+int install_mask(eup_handle* h, uint32_t* bits, int wpr, int64_t nsolid) {
     const Geo& g = h->g;
     if (nsolid <= 0 && bits) { cudaFree(bits); bits = nullptr; }
-    uint8_t* d_flags = nullptr;
     int32_t* blist = nullptr;
-    uint64_t* blinks = nullptr;
+    int64_t nblist = 0;
+    LinksDevice links;
     if (nsolid > 0) {
-        cudaError_t e = cudaMalloc(&d_flags, g.N);
-        if (e == cudaSuccess) e = cudaMalloc(&blist, sizeof(int32_t) * (size_t)nsolid);
-        if (e == cudaSuccess) e = cudaMalloc(&blinks, sizeof(uint64_t) * (size_t)nsolid);
+        // flags, link words and compaction scratch share the staging buffer, which the next
+        // state transfer of this precision needs at its full size anyway
+        const size_t flags_bytes = ((size_t)g.N + 255) / 256 * 256;
+        const size_t words_bytes = (sizeof(uint64_t) * (size_t)nsolid + 255) / 256 * 256;
+        const size_t want = std::max(flags_bytes + words_bytes + ((size_t)1 << 16),
+                                     (size_t)(g.l + 2) * (g.m + 2) * (g.n + 2) * (h->prec == EUP_FP64 ? 8 : 4));
+        const int rc = ensure_staging(h, want);
+        if (rc) {
+            cudaFree(bits);
+            return rc;
+        }
+        uint8_t* flags = static_cast<uint8_t*>(h->staging);
+        uint64_t* words = reinterpret_cast<uint64_t*>(flags + flags_bytes);
+        void* scratch = flags + flags_bytes + words_bytes;
+        const size_t scratch_bytes = h->staging_bytes - flags_bytes - words_bytes;
+        const Mask mk{bits, wpr};
+        const int bc[6] = {h->cfg.bc[0], h->cfg.bc[1], h->cfg.bc[2], h->cfg.bc[3], h->cfg.bc[4], h->cfg.bc[5]};
+        cudaError_t e = cudaMalloc(&blist, sizeof(int32_t) * (size_t)nsolid);
+        if (e == cudaSuccess) {
+            launch_flag_boundary_solid(g, mk, flags, h->stream);
+            nblist = compact_flags(flags, g.N, blist, scratch, scratch_bytes, h->stream, &e);  // <= nsolid: solids
+        }
+        if (e == cudaSuccess) {
+            launch_bsolid_links(g, mk, bc, blist, nblist, words, h->stream);
+            e = build_links(g, bc, blist, words, nblist, &links, scratch, scratch_bytes, h->stream);
+        }
         if (e != cudaSuccess) {
-            cudaFree(d_flags);
             cudaFree(blist);
-            cudaFree(blinks);
             cudaFree(bits);
             return cuda_fail(h, e, "install obstacles");
         }
     }
-    drop_graphs(h);  // the captured steps hold the old mask and list pointers
+    drop_graphs(h);  // the captured steps hold the old link pointers
     if (h->bits) cudaFree(h->bits);
     if (h->blist) cudaFree(h->blist);
-    if (h->blinks) cudaFree(h->blinks);
+    if (h->links.fluid) cudaFree(const_cast<FluidLink*>(h->links.fluid));
+    if (h->links.halo) cudaFree(const_cast<HaloLink*>(h->links.halo));
     h->bits = bits;
+    h->wpr = wpr;
     h->blist = blist;
-    h->blinks = blinks;
-    h->nblist = 0;
+    h->nblist = nblist;
+    h->links = links;
     h->nsolid = nsolid > 0 ? nsolid : 0;
-    if (nsolid > 0) {
-        launch_flag_boundary_solid(g, make_mask(h), d_flags, h->stream);
-        cudaError_t e;
-        const int64_t cnt = compact_flags(d_flags, g.N, h->blist, h->stream, &e);
-        cudaFree(d_flags);
-        if (e != cudaSuccess) return cuda_fail(h, e, "compact boundary solid list");
-        h->nblist = cnt;  // cnt <= nsolid: the boundary solids are solids
-        const int bc[6] = {h->cfg.bc[0], h->cfg.bc[1], h->cfg.bc[2], h->cfg.bc[3], h->cfg.bc[4], h->cfg.bc[5]};
-        launch_bsolid_links(g, make_mask(h), bc, h->blist, cnt, h->blinks, h->stream);
-    }
     if (h->has_state && !h->pbb) DISPATCH(h, enqueue_drag_only, h);
     CK(h, cudaGetLastError());
     CK(h, cudaStreamSynchronize(h->stream));
@@ -695,14 +708,14 @@ int eup_set_obstacles(eup_handle* h, const int32_t* obs) {
     }
     if ((rc = check_obstacles(h, "eup_set_obstacles", nsolid, on_first, on_last))) return rc;
     CK(h, cudaStreamSynchronize(h->stream));
-    h->wpr = (g.l + 31) / 32;
+    const int wpr = (g.l + 31) / 32;
     uint32_t* bits = nullptr;
     if (nsolid > 0) {
         int32_t* d_obs = nullptr;
         CK(h, cudaMalloc(&d_obs, sizeof(int32_t) * g.N));
         cudaError_t e = cudaMemcpyAsync(d_obs, obs, sizeof(int32_t) * g.N, cudaMemcpyHostToDevice, h->stream);
-        if (e == cudaSuccess) e = cudaMalloc(&bits, sizeof(uint32_t) * (size_t)g.m * g.n * h->wpr);
-        if (e == cudaSuccess) launch_build_mask(d_obs, g, bits, h->wpr, h->stream);
+        if (e == cudaSuccess) e = cudaMalloc(&bits, sizeof(uint32_t) * (size_t)g.m * g.n * wpr);
+        if (e == cudaSuccess) launch_build_mask(d_obs, g, bits, wpr, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
         cudaFree(d_obs);
         if (e != cudaSuccess) {
@@ -710,7 +723,7 @@ int eup_set_obstacles(eup_handle* h, const int32_t* obs) {
             return cuda_fail(h, e, "eup_set_obstacles: mask");
         }
     }
-    return install_mask(h, bits, nsolid);
+    return install_mask(h, bits, wpr, nsolid);
 }
 
 int eup_build_obstacles(eup_handle* h, const eup_geometry* geo) {
@@ -753,8 +766,7 @@ int eup_build_obstacles(eup_handle* h, const eup_geometry* geo) {
         cudaFree(bits);
         return rc;
     }
-    h->wpr = wpr;
-    return install_mask(h, bits, (int64_t)cnt[0]);
+    return install_mask(h, bits, wpr, (int64_t)cnt[0]);
 }
 
 int eup_get_obstacles(eup_handle* h, int32_t* obs, int64_t* nobs) {

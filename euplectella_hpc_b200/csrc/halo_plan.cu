@@ -67,10 +67,10 @@ HaloEdges build_halo_edges(const Geo& g, const int bc[6]) {
         const bool all = b == kHaloFrontFix || b == kHaloEdgeFix;
         st.clear();
         for (int y = 0; y < r.nb; ++y) {
-            // an item reaches an edge line only from the two outermost rows or columns of its range
-            const bool row = all || y < 2 || y >= r.nb - 2;
+            // an item reaches an edge line only from the outermost rows and columns of its range
+            const bool row = all || y == 0 || y == r.nb - 1;
             for (int x = 0; x < r.na; ++x) {
-                if (!row && x >= 2 && x < r.na - 2) x = r.na - 2;
+                if (!row && x > 0) x = r.na - 1;
                 halo_item(rec, b, r.a0 + x, r.b0 + y);
             }
         }

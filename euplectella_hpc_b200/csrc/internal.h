@@ -138,19 +138,56 @@ struct HaloFace {
 HaloFace record_halo_face(const Geo& g, const int bc[6], int block);
 
 // Halo planes of one step (CODE/SRC/bcond.bc.F90) in one launch, or one launch per block of
-// the reference; returns the number of kernels launched.
+// the reference; with `force` its sum too.  Returns the number of kernels launched.
 template <typename S, typename R>
 int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, const HaloEdgesDevice& edges,
-              cudaStream_t st, bool separate = false);
+              cudaStream_t st, bool separate = false, const struct ForceSum* force = nullptr);
 
-// Bounce-back on solid voxels touching fluid/halo (CODE/SRC/bcond.obs.F90) and the
-// FP64 momentum-exchange force of the state it reads, written to
-// series[3*(*d_itime % cap)]; with `advance` the device step counter is incremented.
-// links[t] classifies the 18 neighbours of list[t] (see launch_bsolid_links).
+// ---- bounce-back and momentum-exchange force --------------------------------------------
+// The links of the solid voxels to fluid and to halo nodes, population by population (q
+// outermost, voxels ascending), so that neighbouring threads read and write neighbouring
+// values of one population.
+struct FluidLink {
+    int32_t lin;  // solid voxel
+    uint32_t q;   // population 0..17, kLinkXFirst / kLinkXLast when the voxel lies on x = 1 / x = l
+};
+struct HaloLink {
+    int32_t lin;
+    uint32_t q;
+    int64_t ghost;  // halo value the bounce-back reads
+    int64_t wrap;   // interior fluid node beyond a periodic face, whose value enters the force; -1: none
+};
+constexpr uint32_t kLinkXFirst = 32u, kLinkXLast = 64u, kLinkQ = 31u;
+struct LinksDevice {
+    const FluidLink* fluid = nullptr;
+    const HaloLink* halo = nullptr;
+    int64_t nfluid = 0, nhalo = 0;
+};
+// Builds the links of the n boundary-solid voxels of `list`, classified by `words` (see
+// launch_bsolid_links); allocates out->fluid and out->halo, synchronises st.  scratch: device
+// memory to work in (256-byte aligned), more is allocated where it does not suffice.
+cudaError_t build_links(const Geo& g, const int bc[6], const int32_t* list, const uint64_t* words, int64_t n,
+                        LinksDevice* out, void* scratch, size_t scratch_bytes, cudaStream_t st);
+
+// Where a sum of the force goes: series[3 * (*d_itime % cap)]; `blocks` partial sums of the
+// bounce-back launch are added in their order, and the device step counter advances.
+struct ForceSum {
+    const double* partials;
+    int blocks;
+    double* series;
+    int64_t cap;
+    int64_t* d_itime;
+};
+// Bounce-back on solid voxels touching fluid/halo (CODE/SRC/bcond.obs.F90) with partial sums of
+// the FP64 momentum-exchange force of the state it reads; the halo launch of the step adds
+// them (launch_bc with the ForceSum returned).  No launch without links (blocks = 0).
 template <typename S, typename R>
-void launch_bounce_drag(const Lat<S, R>& L, const Geo& g, const int bc[6], const int32_t* list,
-                        const uint64_t* links, int64_t nlist, bool do_bounce, const Reduce& red, double* series,
-                        int64_t cap, int64_t* d_itime, bool advance, cudaStream_t st);
+ForceSum launch_bounce(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
+                       int64_t cap, int64_t* d_itime, cudaStream_t st);
+// The force alone, of the state in L, in one launch; the step counter stays.
+template <typename S, typename R>
+void launch_force(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
+                  int64_t cap, int64_t* d_itime, cudaStream_t st);
 
 // x-slab faces: the five populations crossing an x face, (m+2)(n+2) values each.
 template <typename S, typename R>
@@ -237,7 +274,8 @@ void launch_links(const Geo& g, const Mask& mk, uint32_t* links, cudaStream_t st
 void launch_bsolid_links(const Geo& g, const Mask& mk, const int bc[6], const int32_t* list, int64_t n,
                          uint64_t* links, cudaStream_t st);
 // Ordered compaction of flagged linear indices; returns the count (synchronous).
-int64_t compact_flags(const uint8_t* flags, int64_t n, int32_t* out, cudaStream_t st, cudaError_t* err);
+int64_t compact_flags(const uint8_t* flags, int64_t n, int32_t* out, void* scratch, size_t scratch_bytes,
+                      cudaStream_t st, cudaError_t* err);
 
 // ---- partial bounce-back and its adjoint (k_adjoint.cu) -------------------------
 // Where the adjoint of each halo value goes, derived on the host by running the

@@ -13,13 +13,143 @@ namespace {
 
 constexpr int kTpb = 256;
 
+// ---- bounce-back + momentum exchange ---------------------------------------------------
+//
+// For each solid voxel x touching fluid or halo and each moving q, the
+// reference sets a_q(x) = a_opp(q)(x + c_q) (CODE/SRC/bcond.obs.F90:56-73), so
+// that the next pull returns to the fluid node x + c_q its own post-collision
+// population.  Links whose neighbour is itself solid are skipped: their value
+// is only ever pulled into solid voxels.  The same reads give the force: the
+// population a_opp(q)(y) leaving fluid node y = x + c_q towards x transfers
+// 2 c_opp(q) a_opp(q)(y) = -2 c_q a_opp(q)(y); across a periodic axis y is the
+// wrapped node and its interior value is used.
+//
+// One thread per link.  Like the halo this is a short kernel bound by latency and instruction
+// fetch, so a link is a few instructions with the population's pointers and weights in the
+// parameter bank, the halo links have their source slots in the list, and the partial forces
+// are added by the halo launch that follows instead of by the last block behind a fence and an
+// atomic.  Bounce-back and force of a step (CUDA events, launch included), one thread per voxel
+// with its 18 directions written out and the sum in the kernel / this: 14.4 / 7.0 us at 64x32x8,
+// 16.6 / 8.7 us at 256x128x64, 18.7 / 14.9 us at 768x384x384 FP32.
+template <typename S, typename R>
+struct BounceArgs {
+    Lat<S, R> L;
+    Geo g;
+    LinksDevice links;
+    const S* from[18];  // population opp(q), moved so that the solid voxel's index reads x + c_q
+    R w[18];
+    double c2[18][3];   // -2 c_q
+    double* partials;
+    int bounce;         // store, or the force alone
+    int finish;         // the last block adds the partial sums (series, cap, d_itime)
+    unsigned int* counter;
+    ForceSum sum;
+};
+
+// Sum over the block in threads 0..2 (component = thread); kTpb threads, fixed order.
+__device__ __forceinline__ double block_sum3(double (&f)[3]) {
+    __shared__ double sh[kTpb / 32][3];
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+        f[0] += __shfl_down_sync(0xffffffffu, f[0], o);
+        f[1] += __shfl_down_sync(0xffffffffu, f[1], o);
+        f[2] += __shfl_down_sync(0xffffffffu, f[2], o);
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        sh[threadIdx.x >> 5][0] = f[0];
+        sh[threadIdx.x >> 5][1] = f[1];
+        sh[threadIdx.x >> 5][2] = f[2];
+    }
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x < 3)
+#pragma unroll
+        for (int w = 0; w < kTpb / 32; ++w) s += sh[w][threadIdx.x];
+    return s;
+}
+
+// One block: the partial forces in a fixed order into the force history.
+__device__ __forceinline__ void sum_partials(const ForceSum& a, bool advance) {
+    const int64_t t = *a.d_itime;
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < a.blocks; b += kTpb) {
+        f[0] += __ldcg(a.partials + 3 * b);
+        f[1] += __ldcg(a.partials + 3 * b + 1);
+        f[2] += __ldcg(a.partials + 3 * b + 2);
+    }
+    const double s = block_sum3(f);  // every thread has read d_itime before thread 0 writes it
+    if (threadIdx.x < 3) a.series[3 * (t % a.cap) + threadIdx.x] = s;
+    if (advance && threadIdx.x == 0) *a.d_itime = t + 1;
+}
+
+template <typename S, typename R>
+__global__ void __launch_bounds__(kTpb) k_bounce(const __grid_constant__ BounceArgs<S, R> p) {
+    double f[3] = {0.0, 0.0, 0.0};
+    const int64_t total = p.links.nfluid + p.links.nhalo;
+    for (int64_t t = (int64_t)blockIdx.x * kTpb + threadIdx.x; t < total; t += (int64_t)gridDim.x * kTpb) {
+        int32_t lin;
+        uint32_t e;
+        S raw;
+        R val, push;  // the value stored, and the one that pushes the solid
+        bool counts = true;
+        if (t < p.links.nfluid) {
+            const FluidLink k = p.links.fluid[t];
+            lin = k.lin;
+            e = k.q;
+            raw = p.from[e & kLinkQ][lin];
+            if constexpr (DevStore<S>::value) val = p.w[e & kLinkQ] + DevStore<S>::to_f(raw) * p.L.inv_scale;
+            else val = raw;
+            push = val;
+        } else {
+            const HaloLink k = p.links.halo[t - p.links.nfluid];
+            lin = k.lin;
+            e = k.q;
+            const int q = e & kLinkQ;
+            raw = Store<S, R>::store(p.L.ghost[k.ghost], q, p.L.scale);
+            val = Store<S, R>::load(raw, q, p.L.inv_scale);
+            counts = k.wrap >= 0;
+            push = R(0);
+            if (counts) push = Store<S, R>::load(p.L.pop[opp_of(q)][k.wrap], q, p.L.inv_scale);
+        }
+        const int q = e & kLinkQ;
+        if (p.bounce) {
+            p.L.pop[q][lin] = raw;
+            if (e > kLinkQ) {  // a column the x-face copy holds
+                R* x = p.L.xface + (p.g.xr + xface_slot(q) * p.g.mn + lin / p.g.l);
+                if (e & kLinkXFirst) x[0] = val;
+                if (e & kLinkXLast) x[p.g.xs] = val;
+            }
+        }
+        if (counts) {
+            const double v = (double)push;
+            f[0] += p.c2[q][0] * v;
+            f[1] += p.c2[q][1] * v;
+            f[2] += p.c2[q][2] * v;
+        }
+    }
+    const double s = block_sum3(f);
+    if (threadIdx.x < 3) p.partials[3 * (int64_t)blockIdx.x + threadIdx.x] = s;
+    if (!p.finish) return;
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(p.counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    sum_partials(p.sum, false);
+    if (threadIdx.x == 0) *p.counter = 0u;
+}
+
 // ---- halo planes ---------------------------------------------------------------------
 //
 // One launch for the halo of a step.  A segment is a run of thread blocks with one job: a face
 // (one thread per node of the face, five populations each) or the edge stores of one of the
 // reference's blocks (one thread per store).  The x faces read the compact x-face copy written
 // by the stream-collide kernel (coalesced in j; a strided read of a column costs a sector per
-// node), the others the lattice.
+// node), the others the lattice.  One more thread block adds the partial forces of the
+// bounce-back launch.
 //
 // What bounds it on all but the largest lattices is the latency of a short kernel, and there
 // instruction fetch: a launch starts with cold instruction caches, and ncu puts 80 % of the
@@ -29,7 +159,7 @@ constexpr int kTpb = 256;
 // launch included), as eight dependent launches / as one: 38 / 6.9 us at 64x32x8, 41 / 8.4 us at
 // 256x128x64, 48 / 10.6 us at 384x192x192, 61 / 19.4 us at 768x384x384 FP32.  (One launch with
 // the items' conditions written out: 12 and 23 us at the first two.)
-constexpr int kHaloSegments = 2 * kHaloBlocks;
+constexpr int kHaloSegments = 2 * kHaloBlocks;  // six faces, eight blocks' edges, the force
 
 template <typename S, typename R>
 struct HaloSegment {
@@ -46,7 +176,7 @@ struct HaloSegment {
     R* pass_dst;
     const HaloEdge* edges;
 };
-constexpr int kSegEdges = 100;
+constexpr int kSegEdges = 100, kSegForce = 101;
 
 template <typename S, typename R>
 struct HaloPlan {
@@ -54,6 +184,7 @@ struct HaloPlan {
     Geo g;
     R force;
     R inflow[5];
+    ForceSum sum;
     unsigned first[kHaloSegments + 1];  // first thread block of each segment
     HaloSegment<S, R> seg[kHaloSegments];
 };
@@ -75,6 +206,10 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
     const HaloSegment<S, R>& f = p.seg[s];
     const unsigned t = (blockIdx.x - p.first[s]) * kTpb + threadIdx.x;
     if (t >= f.count) return;
+    if (f.kind == kSegForce) {
+        sum_partials(p.sum, true);
+        return;
+    }
     R v[5];
     if (f.kind == kSegEdges) {
         const HaloEdge e = f.edges[t];
@@ -121,91 +256,6 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
 #pragma unroll
     for (int c = 0; c < 5; ++c)
         if (a + f.da[c] < f.na && b + f.db[c] < f.nb) f.dst[c][to] = v[c];
-}
-
-// ---- bounce-back + momentum exchange ---------------------------------------------------
-//
-// For each solid voxel x touching fluid or halo and each moving q, the
-// reference sets a_q(x) = a_opp(q)(x + c_q) (CODE/SRC/bcond.obs.F90:56-73), so
-// that the next pull returns to the fluid node x + c_q its own post-collision
-// population.  Links whose neighbour is itself solid are skipped: their value
-// is only ever pulled into solid voxels.  The same reads give the force: the
-// population a_opp(q)(y) leaving fluid node y = x + c_q towards x transfers
-// 2 c_opp(q) a_opp(q)(y) = -2 c_q a_opp(q)(y); across a periodic axis y is the
-// wrapped node and its interior value is used.  The force of the state read
-// goes to series[itime % cap], itime read from device memory; with `advance`
-// the last block then increments the device step counter.
-
-template <typename S, typename R>
-__global__ void k_bounce_drag(Lat<S, R> L, Geo g, int per_x, int per_y, int per_z, const int32_t* list,
-                              const uint64_t* links, int64_t nlist, int do_bounce, Reduce red, double* series,
-                              int64_t cap, int64_t* d_itime, int advance) {
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nlist;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t lin = list[t];
-        const uint64_t w = links[t];
-        const uint32_t fl = (uint32_t)(w & 0x3FFFFu);          // neighbour x + c_q is interior fluid
-        const uint32_t gh = (uint32_t)((w >> 18) & 0x3FFFFu);  // neighbour is a halo node
-        const uint32_t wf = (uint32_t)((w >> 36) & 0x3FFFFu);  // halo neighbour wraps onto interior fluid
-        const int i = lin % g.l + 1;
-        const int jk = lin / g.l;
-        const int j = jk % g.m + 1, k = jk / g.m + 1;
-        S raw[18];
-        R val[18];
-        // all loads first: interior fluid neighbours from the lattice, halo ones from the shell
-#pragma unroll
-        for (int q = 0; q < 18; ++q) {
-            const int qo = opp_of(q);
-            raw[q] = S();
-            if ((fl >> q) & 1u) {
-                raw[q] = L.pop[qo][(int64_t)lin + cx_of(q) + (int64_t)cy_of(q) * g.l + (int64_t)cz_of(q) * g.lm];
-            } else if ((gh >> q) & 1u) {
-                const R v = L.ghost[(int64_t)qo * g.G + g.gidx(i + cx_of(q), j + cy_of(q), k + cz_of(q))];
-                raw[q] = Store<S, R>::store(v, q, L.scale);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 18; ++q) {
-            val[q] = ((fl >> q) & 1u) ? Store<S, R>::load(raw[q], opp_of(q), L.inv_scale)
-                                      : Store<S, R>::load(raw[q], q, L.inv_scale);
-            if ((fl >> q) & 1u) {
-                const double v = (double)val[q];
-                f[0] -= 2.0 * cx_of(q) * v;
-                f[1] -= 2.0 * cy_of(q) * v;
-                f[2] -= 2.0 * cz_of(q) * v;
-            }
-        }
-        if (wf) {  // links across a periodic axis: force from the wrapped fluid node
-#pragma unroll
-            for (int q = 0; q < 18; ++q) {
-                if (!((wf >> q) & 1u)) continue;
-                int wi = i + cx_of(q), wj = j + cy_of(q), wk = k + cz_of(q);
-                if (per_x) wi = wi < 1 ? wi + g.l : (wi > g.l ? wi - g.l : wi);
-                if (per_y) wj = wj < 1 ? wj + g.m : (wj > g.m ? wj - g.m : wj);
-                if (per_z) wk = wk < 1 ? wk + g.n : (wk > g.n ? wk - g.n : wk);
-                const double v = (double)lat_load(L, g, opp_of(q), wi, wj, wk);
-                f[0] -= 2.0 * cx_of(q) * v;
-                f[1] -= 2.0 * cy_of(q) * v;
-                f[2] -= 2.0 * cz_of(q) * v;
-            }
-        }
-        if (do_bounce) {
-            const uint32_t wr = fl | gh;
-#pragma unroll
-            for (int q = 0; q < 18; ++q)
-                if ((wr >> q) & 1u) L.pop[q][lin] = raw[q];
-            if (i == 1 || i == g.l) {
-#pragma unroll
-                for (int q = 0; q < 18; ++q) {
-                    if (!((wr >> q) & 1u)) continue;
-                    if (i == 1) L.xface[xface_idx(g, 0, q, j, k)] = val[q];
-                    if (i == g.l) L.xface[xface_idx(g, 1, q, j, k)] = val[q];
-                }
-            }
-        }
-    }
-    block_reduce_store<3>(f, red, nullptr, series, cap, d_itime, advance);
 }
 
 // ---- FP64 monitor, CODE/SRC/diagno.F90:67-120 -------------------------------------------
@@ -603,7 +653,7 @@ void launch_unpack_x(const Lat<S, R>& L, const Geo& g, int side, const R* in, cu
 
 template <typename S, typename R>
 int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, const HaloEdgesDevice& edges,
-              cudaStream_t st, bool separate) {
+              cudaStream_t st, bool separate, const ForceSum* force) {
     HaloPlan<S, R> p{};
     p.L = L;
     p.g = g;
@@ -617,14 +667,23 @@ int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& 
         k_halo<S, R><<<blocks, kTpb, 0, st>>>(p);
         ++launches;
         n = 0;
+        p.first[0] = 0;
     };
     auto add = [&](const HaloSegment<S, R>& f) {
         p.seg[n] = f;
         p.first[n + 1] = p.first[n] + (f.count + kTpb - 1) / kTpb;
         ++n;
     };
+    p.first[0] = 0;
+    if (force) {
+        p.sum = *force;
+        HaloSegment<S, R> f{};
+        f.kind = kSegForce;
+        f.count = kTpb;
+        add(f);
+    }
     for (int b = 0; b < kHaloBlocks; ++b) {
-        p.first[0] = 0;
+        const int before = n;
         const HaloFace face = record_halo_face(g, bc, b);
         if (face.kind != kFaceNone) {
             HaloSegment<S, R> f{};
@@ -658,21 +717,50 @@ int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& 
             f.edges = edges.e + edges.first[b];
             add(f);
         }
-        if (separate) launch();
+        if (separate && n > before) launch();
     }
     launch();
     return launches;
 }
 
 template <typename S, typename R>
-void launch_bounce_drag(const Lat<S, R>& L, const Geo& g, const int bc[6], const int32_t* list,
-                        const uint64_t* links, int64_t nlist, bool do_bounce, const Reduce& red, double* series,
-                        int64_t cap, int64_t* d_itime, bool advance, cudaStream_t st) {
-    const int per_x = (bc[0] == 0 && bc[1] == 0), per_y = (bc[2] == 0 && bc[3] == 0);
-    const int per_z = (bc[4] == 0 && bc[5] == 0);
-    const unsigned blocks = grid_for(nlist, kTpb, (unsigned)red.max_blocks);
-    k_bounce_drag<S, R><<<blocks, kTpb, 0, st>>>(L, g, per_x, per_y, per_z, list, links, nlist, do_bounce ? 1 : 0,
-                                                 red, series, cap, d_itime, advance ? 1 : 0);
+BounceArgs<S, R> bounce_args(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red) {
+    BounceArgs<S, R> p{};
+    p.L = L;
+    p.g = g;
+    p.links = links;
+    for (int q = 0; q < 18; ++q) {
+        p.from[q] = L.pop[opp_of(q)] + (cx_of(q) + (int64_t)cy_of(q) * g.l + (int64_t)cz_of(q) * g.lm);
+        p.w[q] = wclass_of(q) == 1 ? R(1.0 / 18.0) : R(1.0 / 36.0);
+        p.c2[q][0] = -2.0 * cx_of(q);
+        p.c2[q][1] = -2.0 * cy_of(q);
+        p.c2[q][2] = -2.0 * cz_of(q);
+    }
+    p.partials = red.partials;
+    p.counter = red.counter;
+    return p;
+}
+
+template <typename S, typename R>
+ForceSum launch_bounce(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
+                       int64_t cap, int64_t* d_itime, cudaStream_t st) {
+    ForceSum sum{red.partials, 0, series, cap, d_itime};
+    if (links.nfluid + links.nhalo == 0) return sum;
+    BounceArgs<S, R> p = bounce_args(L, g, links, red);
+    p.bounce = 1;
+    sum.blocks = (int)grid_for(links.nfluid + links.nhalo, kTpb, (unsigned)red.max_blocks);
+    k_bounce<S, R><<<(unsigned)sum.blocks, kTpb, 0, st>>>(p);
+    return sum;
+}
+
+template <typename S, typename R>
+void launch_force(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
+                  int64_t cap, int64_t* d_itime, cudaStream_t st) {
+    BounceArgs<S, R> p = bounce_args(L, g, links, red);
+    p.finish = 1;
+    p.sum = ForceSum{red.partials, (int)grid_for(links.nfluid + links.nhalo, kTpb, (unsigned)red.max_blocks), series,
+                     cap, d_itime};
+    k_bounce<S, R><<<(unsigned)p.sum.blocks, kTpb, 0, st>>>(p);
 }
 
 template <typename S, typename R>
@@ -744,10 +832,11 @@ void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStre
 
 #define EUP_INST(S, R)                                                                                 \
     template int launch_bc<S, R>(const Lat<S, R>&, const Geo&, const int*, const Phys<R>&, const HaloEdgesDevice&, \
-                                 cudaStream_t, bool);                                                     \
-    template void launch_bounce_drag<S, R>(const Lat<S, R>&, const Geo&, const int*, const int32_t*,   \
-                                           const uint64_t*, int64_t, bool, const Reduce&, double*,     \
-                                           int64_t, int64_t*, bool, cudaStream_t);                     \
+                                 cudaStream_t, bool, const ForceSum*);                                    \
+    template ForceSum launch_bounce<S, R>(const Lat<S, R>&, const Geo&, const LinksDevice&, const Reduce&, double*, \
+                                          int64_t, int64_t*, cudaStream_t);                            \
+    template void launch_force<S, R>(const Lat<S, R>&, const Geo&, const LinksDevice&, const Reduce&, double*, \
+                                     int64_t, int64_t*, cudaStream_t);                                 \
     template void launch_fill_xface<S, R>(const Lat<S, R>&, const Geo&, cudaStream_t);                 \
     template void launch_pack_x<S, R>(const Lat<S, R>&, const Geo&, int, R*, cudaStream_t);              \
     template void launch_unpack_x<S, R>(const Lat<S, R>&, const Geo&, int, const R*, cudaStream_t);      \
