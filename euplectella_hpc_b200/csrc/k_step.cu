@@ -5,6 +5,8 @@
 // Nodes whose 18 upstream neighbours are all interior take the fast path
 // (plain shifted loads); nodes on the six boundary planes resolve each pull
 // through the halo shell.
+#include <string.h>
+
 #include "internal.h"
 
 namespace eup {
@@ -39,16 +41,30 @@ struct KOps {
     }
 };
 
+// Whether the row (j - cy, k - cz) that population q is pulled from lies on a y or z halo
+// plane, and where it starts in the shell then (*row: the element of x = 1; an x plane's element
+// only ever replaces the end values of a row).  j and k belong to the row, so this is
+// uniform over a block of the row kernels; rows away from the boundary planes never ask.
+template <typename R>
+__device__ __forceinline__ bool halo_row(const R* ghost, const Geo& g, int q, int j, int k, const R** row) {
+    const int cy = cy_of(q), cz = cz_of(q);
+    const bool oy = cy == 1 ? j == 1 : (cy == -1 ? j == g.m : false);
+    const bool oz = cz == 1 ? k == 1 : (cz == -1 ? k == g.n : false);
+    const int64_t y = (cy == 1 ? g.oy0 : g.oym) + (int64_t)(k - cz) * g.l;
+    const int64_t z = (cz == 1 ? g.oz0 : g.ozn) + (int64_t)(j - cy - 1) * g.l;
+    *row = ghost + ((int64_t)q * g.G + (oy ? y : z));
+    return oy | oz;
+}
+
 // Streamed populations of interior node (i, j, k); rowlin = l*((j-1) + m*(k-1))
 // is the linear index of x = 1 on its row (32-bit: one lattice holds fewer than
 // 2^31 nodes).  Every source row pointer depends on the row only, so it is the
 // same for the whole warp and each load is that pointer plus the thread's x.
-// Rows on the y/z boundary planes (warp-uniform) resolve every pull through
-// the halo shell.  Elsewhere all 18 shifted loads are issued unconditionally --
-// for such rows every shifted index stays inside [0, N): D3Q19 has no (1,1,1)
-// diagonals, so x = 0 of row (j', k') is x = l of row (j'-1, k') with j' >= 1,
-// k' >= 2 or j' >= 2 -- and the five x-halo values of the first/last node of a
-// row replace them afterwards.
+// All 18 shifted loads are issued unconditionally, and the five x-halo values of
+// the first/last node of a row replace them afterwards: a shifted index off the end
+// of a row reads the neighbouring row, the population's padding, or on a halo row the
+// neighbouring element of the shell.  A row on the y/z boundary planes pulls some
+// populations from halo rows instead (halo_row): only the pointers differ.
 template <typename S, typename R>
 __device__ __forceinline__ void gather_node(const Lat<S, R>& src, const Geo& g, int i, int j, int k, int rowlin,
                                             R (&x)[19]) {
@@ -61,22 +77,41 @@ __device__ __forceinline__ void gather_node(const Lat<S, R>& src, const Geo& g, 
             const S* rp = src.pop[q] + (rowlin - cy_of(q) * l - cz_of(q) * lm);
             x[q] = K::val(rp[i - 1 - cx_of(q)], q, src);
         }
-        if (i == 1) {
+    } else if constexpr (!K::dev) {
 #pragma unroll
-            for (int q = 0; q < 18; ++q)
-                if (cx_of(q) == 1)
-                    x[q] = K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(0, j - cy_of(q), k - cz_of(q))], q, src);
+        for (int q = 0; q < 18; ++q) {
+            const R* halo;
+            const bool out = halo_row(src.ghost, g, q, j, k, &halo);
+            const S* rp = out ? halo : src.pop[q] + (rowlin - cy_of(q) * l - cz_of(q) * lm);
+            x[q] = rp[i - 1 - cx_of(q)];
         }
-        if (i == l) {
+    } else {  // lattice and shell hold different types: both loads, one of them at a place that is there
+        S raw[18];
+        R f[18];
 #pragma unroll
-            for (int q = 0; q < 18; ++q)
-                if (cx_of(q) == -1)
-                    x[q] = K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(l + 1, j - cy_of(q), k - cz_of(q))], q,
-                                         src);
+        for (int q = 0; q < 18; ++q) {
+            const R* halo;
+            const bool out = halo_row(src.ghost, g, q, j, k, &halo);
+            raw[q] = (src.pop[q] + (out ? rowlin : rowlin - cy_of(q) * l - cz_of(q) * lm))[i - 1 - cx_of(q)];
+            f[q] = (out ? halo : src.ghost)[out ? i - 1 - cx_of(q) : 0];
         }
-    } else {
 #pragma unroll
-        for (int q = 0; q < 18; ++q) x[q] = K::pull(src, g, q, i - cx_of(q), j - cy_of(q), k - cz_of(q));
+        for (int q = 0; q < 18; ++q) {
+            const R* halo;
+            x[q] = halo_row(src.ghost, g, q, j, k, &halo) ? K::from_shell(f[q], q, src) : K::val(raw[q], q, src);
+        }
+    }
+    if (i == 1) {
+#pragma unroll
+        for (int q = 0; q < 18; ++q)
+            if (cx_of(q) == 1)
+                x[q] = K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(0, j - cy_of(q), k - cz_of(q))], q, src);
+    }
+    if (i == l) {
+#pragma unroll
+        for (int q = 0; q < 18; ++q)
+            if (cx_of(q) == -1)
+                x[q] = K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(l + 1, j - cy_of(q), k - cz_of(q))], q, src);
     }
     x[18] = K::val(src.pop[18][rowlin + i - 1], 18, src);
 }
@@ -168,19 +203,6 @@ template <> struct Vec2<__nv_bfloat16> {
     static __device__ __forceinline__ __nv_bfloat16 hi(__nv_bfloat162 v) { return __high2bfloat16(v); }
 };
 
-// The two nodes of a y/z boundary row (warp-uniform), one by one through the halo shell.
-template <typename S>
-__device__ __forceinline__ void pair_through_shell(const Lat<S, float>& src, const Lat<S, float>& dst, const Geo& g,
-                                                   const Phys<float>& ph, int i, int j, int k, int rowlin) {
-#pragma unroll 1
-    for (int e = 0; e < 2; ++e) {
-        float x[19];
-        gather_node(src, g, i + e, j, k, rowlin, x);
-        KOps<S, float>::collide_node(x, ph, src);
-        scatter_node(dst, g, i + e, j, k, rowlin, x);
-    }
-}
-
 // Population q's source pointer moved back by c_q: the pull a_q(x - c_q) of node index x
 // (0-based, x = i-1 + l (j-1 + m (k-1))) is base[q][x].  Set on the host per launch.
 template <typename S>
@@ -251,8 +273,13 @@ __device__ __forceinline__ void finish_pair(const Lat<S, float>& src, const Lat<
     }
 }
 
-// The pair (i, i+1) of row (j, k).  Rows on the y/z boundary planes go node by node
-// through the halo shell (warp-uniform in the row kernel, where a block is one row).
+// The pair (i, i+1) of row (j, k).  A row on the y/z boundary planes (warp-uniform in the row
+// kernel, where a block is one row) takes the populations that halo_row names from the shell;
+// FP32 rows of both kinds share the collision and the stores.  (With the boundary rows node by
+// node through the shell these rows took 12 us each, whatever the lattice: all of a 64x32x8
+// step's kernel, and the tail of a larger one's, whose last rows are the plane k = n.  Per
+// launch, before / now, CUDA events: 64x32x8 FP32 11.6 / 7.5 us, FP16 16.0 / 9.9; 256x128x64
+// FP32 61.8 / 58.5, FP16 56 / 44.5; 768x384x384 FP32 2656 / 2645, FP16 1690 / 1664.)
 template <typename S>
 __device__ __forceinline__ void pair_step(const Lat<S, float>& src, const Lat<S, float>& dst, const Geo& g,
                                           const Phys<float>& ph, const PullBase<S>& pb, int i, int j, int k) {
@@ -263,12 +290,55 @@ __device__ __forceinline__ void pair_step(const Lat<S, float>& src, const Lat<S,
     const int l = g.l, lm = (int)g.lm;
     const int rowlin = l * ((j - 1) + g.m * (k - 1));
     const bool face_yz = (j == 1) | (j == g.m) | (k == 1) | (k == g.n);
-    if (face_yz) {
-        pair_through_shell(src, dst, g, ph, i, j, k, rowlin);
-        return;
-    }
     F2 x[19];
-    if constexpr (dev) {
+    if (face_yz) {
+        if constexpr (dev) {
+            // one 4-byte load from the lattice (both nodes) or two from the shell, one per node;
+            // a lattice row repeats its load.  By groups, so that the raw words of a few
+            // populations are live beside the values of the others.
+            const uint32_t n0 = (uint32_t)(rowlin + i - 1);
+            constexpr int kGroup = 9;
+#pragma unroll
+            for (int q0 = 0; q0 < 18; q0 += kGroup) {
+                uint32_t a[kGroup], b[kGroup];
+#pragma unroll
+                for (int c = 0; c < kGroup; ++c) {
+                    const int q = q0 + c;
+                    const float* halo;
+                    const bool out = halo_row(src.ghost, g, q, j, k, &halo);
+                    const void* p = out ? static_cast<const void*>(halo + (i - 1 - cx_of(q)))
+                                        : static_cast<const void*>(pb.p[q] + n0);
+                    a[c] = static_cast<const uint32_t*>(p)[0];
+                    b[c] = static_cast<const uint32_t*>(p)[out ? 1 : 0];
+                }
+#pragma unroll
+                for (int c = 0; c < kGroup; ++c) {
+                    const int q = q0 + c;
+                    const float* halo;
+                    if (halo_row(src.ghost, g, q, j, k, &halo)) {
+                        x[q] = F2(K::from_shell(__uint_as_float(a[c]), q, src),
+                                  K::from_shell(__uint_as_float(b[c]), q, src));
+                    } else {
+                        T2 r;
+                        memcpy(&r, &a[c], 4);
+                        x[q] = F2(V2::unpack(r));
+                    }
+                }
+            }
+            x[18] = F2(V2::unpack(*reinterpret_cast<const T2*>(pb.p[18] + n0)));
+            finish_pair(src, dst, g, ph, i, j, k, rowlin, x);
+            return;  // its own collision: sharing the one below costs it 2 % at 1024x512x512
+        } else {
+#pragma unroll
+            for (int q = 0; q < 18; ++q) {
+                const float* halo;
+                const bool out = halo_row(src.ghost, g, q, j, k, &halo);
+                const S* rp = out ? halo : src.pop[q] + (rowlin - cy_of(q) * l - cz_of(q) * lm);
+                x[q] = F2(rp[i - 1 - cx_of(q)], rp[i - cx_of(q)]);
+            }
+            x[18] = F2(src.pop[18][rowlin + i - 1], src.pop[18][rowlin + i]);
+        }
+    } else if constexpr (dev) {
         T2 r[19];
         load_pair_raw(pb, i, rowlin, r);
 #pragma unroll
@@ -282,7 +352,7 @@ __device__ __forceinline__ void pair_step(const Lat<S, float>& src, const Lat<S,
                 const float2 v = V2::unpack(*reinterpret_cast<const T2*>(rp + (i - 1)));
                 x[q] = F2(K::val(v.x, q, src), K::val(v.y, q, src));
             } else {
-                // both shifted loads are in bounds (interior rows; see gather_node)
+                // both shifted loads are in bounds (see gather_node)
                 x[q] = F2(K::val(rp[i - 1 - cx], q, src), K::val(rp[i - cx], q, src));
             }
         }
