@@ -447,7 +447,7 @@ class Solver:
     def region_sums(self, region) -> np.ndarray:
         """FP64 {count, sum rho, sum ux, sum uy, sum uz, sum u^2} over the fluid nodes where
         region (shape (n, m, l), truthy = included) is set."""
-        r = np.ascontiguousarray(np.asarray(region, dtype=bool).astype(np.uint8))
+        r = np.ascontiguousarray(region, dtype=bool).view(np.uint8)
         assert r.shape == (self.cfg.lz, self.cfg.ly, self.cfg.lx)
         out = np.zeros(6, dtype=np.float64)
         self._ck(lib.eup_get_region_sums(self._h, r.ctypes.data, out.ctypes.data))

@@ -349,8 +349,8 @@ void line_dispatch(eup_handle* h, int axis, int c1, int c2, double* d_out) {
     launch_line<S, R>(make_lat<S, R>(h, h->cur), h->g, axis, c1, c2, d_out, h->stream);
 }
 template <typename S, typename R>
-void plane_dispatch(eup_handle* h, int axis, double* d_out) {
-    launch_plane_means<S, R>(make_lat<S, R>(h, h->cur), h->g, axis, d_out, h->stream);
+void plane_dispatch(eup_handle* h, int axis, double* d_out, double* scratch) {
+    launch_plane_means<S, R>(make_lat<S, R>(h, h->cur), h->g, axis, d_out, scratch, h->stream);
 }
 template <typename S, typename R>
 void cv_dispatch(eup_handle* h, const int* box) {
@@ -1216,8 +1216,9 @@ int eup_get_plane_means(eup_handle* h, int32_t axis, double* out) {
     if (!out || axis < 0 || axis > 2) return fail(h, EUP_ERR_INVALID_ARG, "eup_get_plane_means: bad axis or null out");
     if (!h->has_state) return fail(h, EUP_ERR_INVALID_ARG, "eup_get_plane_means: no state uploaded");
     const int len = axis == 0 ? g.l : (axis == 1 ? g.m : g.n);
-    if ((rc = ensure_staging(h, sizeof(double) * 4 * (size_t)len))) return rc;
-    DISPATCH(h, plane_dispatch, h, axis, static_cast<double*>(h->staging));
+    if ((rc = ensure_staging(h, sizeof(double) * (4 * (size_t)len + (size_t)plane_means_scratch(g, axis))))) return rc;
+    double* sums = static_cast<double*>(h->staging);
+    DISPATCH(h, plane_dispatch, h, axis, sums, sums + 4 * (size_t)len);
     CK(h, cudaGetLastError());
     CK(h, cudaMemcpyAsync(out, h->staging, sizeof(double) * 4 * (size_t)len, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -1259,8 +1260,8 @@ int eup_get_region_sums(eup_handle* h, const uint8_t* region, double out[6]) {
     if (rc) return rc;
     if (!region || !out) return fail(h, EUP_ERR_INVALID_ARG, "eup_get_region_sums: null argument");
     if (!h->has_state) return fail(h, EUP_ERR_INVALID_ARG, "eup_get_region_sums: no state uploaded");
-    uint8_t* d_region = nullptr;
-    CK(h, cudaMalloc(&d_region, (size_t)h->g.N));
+    if ((rc = ensure_staging(h, (size_t)h->g.N))) return rc;
+    uint8_t* d_region = static_cast<uint8_t*>(h->staging);
     cudaError_t e = cudaMemcpyAsync(d_region, region, (size_t)h->g.N, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         DISPATCH(h, region_dispatch, h, d_region);
@@ -1268,7 +1269,6 @@ int eup_get_region_sums(eup_handle* h, const uint8_t* region, double out[6]) {
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, h->dscratch, sizeof(double) * 6, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(d_region);
     if (e != cudaSuccess) return cuda_fail(h, e, "eup_get_region_sums");
     for (int c = 0; c < 6; ++c)
         if (!std::isfinite(out[c])) return fail(h, EUP_ERR_DIVERGED, "eup_get_region_sums: non-finite FP64 sum");
@@ -1284,16 +1284,14 @@ int eup_get_probes(eup_handle* h, int32_t npts, const int32_t* ijk, double* rho_
         if (!h->g.interior(ijk[3 * p], ijk[3 * p + 1], ijk[3 * p + 2]))
             return fail(h, EUP_ERR_INVALID_ARG, "eup_get_probes: probe outside the interior");
     if (npts == 0) return EUP_OK;
-    int32_t* d_ijk = nullptr;
-    double* d_out = nullptr;
-    CK(h, cudaMalloc(&d_ijk, sizeof(int32_t) * 3 * npts));
-    CK(h, cudaMalloc(&d_out, sizeof(double) * 4 * npts));
+    const size_t out_bytes = sizeof(double) * 4 * (size_t)npts;
+    if ((rc = ensure_staging(h, out_bytes + sizeof(int32_t) * 3 * (size_t)npts))) return rc;
+    double* d_out = static_cast<double*>(h->staging);
+    int32_t* d_ijk = reinterpret_cast<int32_t*>(d_out + 4 * (size_t)npts);
     CK(h, cudaMemcpyAsync(d_ijk, ijk, sizeof(int32_t) * 3 * npts, cudaMemcpyHostToDevice, h->stream));
     DISPATCH(h, probes_dispatch, h, npts, d_ijk, d_out);
-    cudaMemcpyAsync(rho_u, d_out, sizeof(double) * 4 * npts, cudaMemcpyDeviceToHost, h->stream);
+    cudaMemcpyAsync(rho_u, d_out, out_bytes, cudaMemcpyDeviceToHost, h->stream);
     cudaError_t e = cudaStreamSynchronize(h->stream);
-    cudaFree(d_ijk);
-    cudaFree(d_out);
     if (e != cudaSuccess) return cuda_fail(h, e, "eup_get_probes");
     return EUP_OK;
 }

@@ -4,6 +4,8 @@
 // (CODE/SRC/probe_global.F90) and the host-layout scatter/gather used by
 // upload and download.  All of it is O(surface) or O(solid surface) work.
 #include "init_eq.h"
+#include <algorithm>
+
 #include "halo.h"
 #include "internal.h"
 
@@ -259,30 +261,49 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
 }
 
 // ---- FP64 monitor, CODE/SRC/diagno.F90:67-120 -------------------------------------------
+//
+// The diagnostics over all nodes walk the lattice by rows along x, a warp to a row: the loads of
+// every population are coalesced, the row index is all the mask needs (32 nodes share a word), and
+// no node pays for a division.  What bounds them is the read of the state, for 4- and 8-byte
+// storage; for 16-bit storage the conversions to FP64 and the FP64 adds.  Monitor, a thread per
+// node with three divisions / a warp per row: 298 / 232 us at 384x192x192 FP32, 2290 / 1560 at
+// 768x384x384, 5.3 / 3.3..3.8 ms at 1024x512x512 FP16.
+
+// Density and momentum of node lin in FP64.
 template <typename S, typename R>
-__global__ void k_monitor(Lat<S, R> L, Geo g, Mask mk, Reduce red, double* out) {
+__device__ __forceinline__ void node_sums(const Lat<S, R>& L, int64_t lin, double& rho, double& xj, double& yj,
+                                          double& zj, double& usq) {
+    S raw[19];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) raw[q] = L.pop[q][lin];
+    double a[19];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) a[q] = (double)Store<S, R>::load(raw[q], q, L.inv_scale);
+    rho = 0.0;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) rho += a[q];
+    const double ri = 1.0 / rho;
+    xj = (a[0] + a[1] + a[2] + a[3] + a[4] - a[9] - a[10] - a[11] - a[12] - a[13]) * ri;
+    yj = (a[2] + a[6] + a[7] + a[8] + a[11] - a[0] - a[9] - a[15] - a[16] - a[17]) * ri;
+    zj = (a[3] + a[5] + a[6] + a[12] + a[17] - a[1] - a[8] - a[10] - a[14] - a[15]) * ri;
+    usq = xj * xj + yj * yj + zj * zj;
+}
+
+template <typename S, typename R>
+__global__ void __launch_bounds__(kTpb) k_monitor(Lat<S, R> L, int l, int64_t rows, Mask mk, Reduce red, double* out) {
     double s[5] = {0, 0, 0, 0, 0};
-    for (int64_t lin = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; lin < g.N;
-         lin += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(lin % g.l) + 1;
-        const int j = (int)((lin / g.l) % g.m) + 1;
-        const int k = (int)(lin / g.lm) + 1;
-        if (mk.solid(g, i, j, k)) {
-            s[0] += 1.0;
-            continue;
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * (kTpb / 32);
+    for (int64_t r = (int64_t)blockIdx.x * (kTpb / 32) + (threadIdx.x >> 5); r < rows; r += step)
+        for (int x = lane; x < l; x += 32) {
+            if (mk.bits != nullptr && (mk.bits[r * mk.wpr + (x >> 5)] >> lane) & 1u) {
+                s[0] += 1.0;
+                continue;
+            }
+            double rho, xj, yj, zj, usq;
+            node_sums(L, r * l + x, rho, xj, yj, zj, usq);
+            s[0] += rho; s[1] += xj; s[2] += yj; s[3] += zj; s[4] += usq;
         }
-        double a[19];
-#pragma unroll
-        for (int q = 0; q < 19; ++q) a[q] = (double)Store<S, R>::load(L.pop[q][lin], q, L.inv_scale);
-        double rho = 0.0;
-#pragma unroll
-        for (int q = 0; q < 19; ++q) rho += a[q];
-        const double ri = 1.0 / rho;
-        const double xj = (a[0] + a[1] + a[2] + a[3] + a[4] - a[9] - a[10] - a[11] - a[12] - a[13]) * ri;
-        const double yj = (a[2] + a[6] + a[7] + a[8] + a[11] - a[0] - a[9] - a[15] - a[16] - a[17]) * ri;
-        const double zj = (a[3] + a[5] + a[6] + a[12] + a[17] - a[1] - a[8] - a[10] - a[14] - a[15]) * ri;
-        s[0] += rho; s[1] += xj; s[2] += yj; s[3] += zj; s[4] += xj * xj + yj * yj + zj * zj;
-    }
     block_reduce_store<5>(s, red, out);
 }
 
@@ -290,27 +311,19 @@ __global__ void k_monitor(Lat<S, R> L, Geo g, Mask mk, Reduce red, double* out) 
 // a probe box, ...): {count, sum rho, sum ux, sum uy, sum uz, sum u^2}, u = j/rho
 // as CODE/SRC/diagno.F90:86-105 computes it.
 template <typename S, typename R>
-__global__ void k_region_sums(Lat<S, R> L, Geo g, Mask mk, const uint8_t* region, Reduce red, double* out) {
+__global__ void __launch_bounds__(kTpb) k_region_sums(Lat<S, R> L, int l, int64_t rows, Mask mk, const uint8_t* region,
+                                                      Reduce red, double* out) {
     double s[6] = {0, 0, 0, 0, 0, 0};
-    for (int64_t lin = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; lin < g.N;
-         lin += (int64_t)gridDim.x * blockDim.x) {
-        if (!region[lin]) continue;
-        const int i = (int)(lin % g.l) + 1;
-        const int j = (int)((lin / g.l) % g.m) + 1;
-        const int k = (int)(lin / g.lm) + 1;
-        if (mk.solid(g, i, j, k)) continue;
-        double a[19];
-#pragma unroll
-        for (int q = 0; q < 19; ++q) a[q] = (double)Store<S, R>::load(L.pop[q][lin], q, L.inv_scale);
-        double rho = 0.0;
-#pragma unroll
-        for (int q = 0; q < 19; ++q) rho += a[q];
-        const double ri = 1.0 / rho;
-        const double xj = (a[0] + a[1] + a[2] + a[3] + a[4] - a[9] - a[10] - a[11] - a[12] - a[13]) * ri;
-        const double yj = (a[2] + a[6] + a[7] + a[8] + a[11] - a[0] - a[9] - a[15] - a[16] - a[17]) * ri;
-        const double zj = (a[3] + a[5] + a[6] + a[12] + a[17] - a[1] - a[8] - a[10] - a[14] - a[15]) * ri;
-        s[0] += 1.0; s[1] += rho; s[2] += xj; s[3] += yj; s[4] += zj; s[5] += xj * xj + yj * yj + zj * zj;
-    }
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * (kTpb / 32);
+    for (int64_t r = (int64_t)blockIdx.x * (kTpb / 32) + (threadIdx.x >> 5); r < rows; r += step)
+        for (int x = lane; x < l; x += 32) {
+            if (!region[r * l + x]) continue;
+            if (mk.bits != nullptr && (mk.bits[r * mk.wpr + (x >> 5)] >> lane) & 1u) continue;
+            double rho, xj, yj, zj, usq;
+            node_sums(L, r * l + x, rho, xj, yj, zj, usq);
+            s[0] += 1.0; s[1] += rho; s[2] += xj; s[3] += yj; s[4] += zj; s[5] += usq;
+        }
     block_reduce_store<6>(s, red, out);
 }
 
@@ -321,9 +334,12 @@ __global__ void k_region_sums(Lat<S, R> L, Geo g, Mask mk, const uint8_t* region
 // CODE/SRC/varm.F90:53-85 (div = false: momentum * (1 / den)).
 template <typename S, typename R>
 __device__ __forceinline__ void ref_macro(const Lat<S, R>& L, int64_t lin, bool div, R& den, R& u, R& w, R& v) {
+    S raw[19];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) raw[q] = L.pop[q][lin];
     R f[19];
 #pragma unroll
-    for (int q = 0; q < 19; ++q) f[q] = Store<S, R>::load(L.pop[q][lin], q, L.inv_scale);
+    for (int q = 0; q < 19; ++q) f[q] = Store<S, R>::load(raw[q], q, L.inv_scale);
     const R r = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8] + f[9] + f[10] + f[11] + f[12] + f[13] +
                 f[14] + f[15] + f[16] + f[17] + f[18];
     const R mx = f[0] + f[1] + f[2] + f[3] + f[4] - f[9] - f[10] - f[11] - f[12] - f[13];
@@ -354,37 +370,67 @@ __global__ void k_line(Lat<S, R> L, Geo g, int axis, int c1, int c2, double* out
     out[4 * (t - 1) + 3] = (double)den;
 }
 
-// One block per plane normal to `axis` (CODE/SRC/varm.F90:42-98 for axis z):
-// FP64 sums of u, w, v (momentum times 1/den in R) and den over the plane's
-// nodes, a fixed thread assignment and tree, then divided by the node count.
-template <typename S, typename R>
-__global__ void k_plane_means(Lat<S, R> L, Geo g, int axis, double* out) {
-    const int pl = blockIdx.x;  // 0-based plane
-    const int64_t cnt = axis == 0 ? (int64_t)g.m * g.n : (axis == 1 ? (int64_t)g.l * g.n : g.lm);
+// Plane means (CODE/SRC/varm.F90:42-98 for axis z): FP64 sums of u, w, v (momentum times 1/den
+// in R) and den over the nodes of each plane, divided by their number, in two passes with a
+// fixed order.  A thread keeps its x and walks rows, so the state is read once and coalesced
+// for every axis: rows of one plane for the planes normal to y and z, with a sum over the block
+// at the end, and a share of all rows for those normal to x, where the thread's column is the
+// plane.  (One block per plane, walked by 256 threads, a row's stride apart for the planes
+// normal to x, took 1110 / 848 / 803 us for the planes normal to x / y / z at 384x192x192 FP32
+// and 27.9 / 6.2 / 5.8 ms at 1024x512x512 FP16; now 200 us and 2.6..3.5 ms.  A warp per row
+// with a sum over its lanes at the end of each: 226 us, 3.5 ms.)
+struct PlaneWalk {
+    int l, rows;          // rows of a plane (all rows for axis 0)
+    int shares, xblocks;  // thread blocks a plane is dealt to, by rows and along x
+    int64_t plane, row;   // row index of row t of plane p: p * plane + t * row
+};
+
+template <typename S, typename R, bool COLUMN>
+__global__ void __launch_bounds__(128) k_plane_sums(Lat<S, R> L, PlaneWalk w, double* part) {
+    const int xb = blockIdx.x % w.xblocks, ps = blockIdx.x / w.xblocks;  // ps = plane * shares + share
+    const int share = ps % w.shares;
+    const int64_t first = (int64_t)(ps / w.shares) * w.plane;
+    const int x = xb * blockDim.x + threadIdx.x;
     double s[4] = {0, 0, 0, 0};
-    for (int64_t t = threadIdx.x; t < cnt; t += blockDim.x) {
-        int64_t lin;
-        if (axis == 2) lin = (int64_t)pl * g.lm + t;
-        else if (axis == 0) lin = pl + (int64_t)g.l * t;                             // t = (j-1) + m (k-1)
-        else lin = (t % g.l) + (int64_t)g.l * (pl + (int64_t)g.m * (t / g.l));       // t = (i-1) + l (k-1)
-        R den, u, w, v;
-        ref_macro(L, lin, false, den, u, w, v);
-        s[0] += (double)u; s[1] += (double)w; s[2] += (double)v; s[3] += (double)den;
-    }
-    __shared__ double sh[32][4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_down_sync(0xffffffffu, s[c], o);
-    if (lane == 0)
-        for (int c = 0; c < 4; ++c) sh[warp][c] = s[c];
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 4; ++c) {
-            double a = 0.0;
-            for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) a += sh[wv][c];
-            out[4 * pl + c] = a / (double)cnt;
+    if (x < w.l)
+        for (int t = share * blockDim.y + threadIdx.y; t < w.rows; t += w.shares * blockDim.y) {
+            R den, u, v, z;
+            ref_macro(L, (first + t * w.row) * w.l + x, false, den, u, v, z);
+            s[0] += (double)u; s[1] += (double)v; s[2] += (double)z; s[3] += (double)den;
         }
+    if constexpr (COLUMN) {  // part[((share * blockDim.y + threadIdx.y) * 4 + c) * l + x]
+        if (x < w.l)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) part[((int64_t)(share * blockDim.y + threadIdx.y) * 4 + c) * w.l + x] = s[c];
+    } else {
+        __shared__ double sh[4][4];
+        const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_down_sync(0xffffffffu, s[c], o);
+        if ((tid & 31) == 0)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) sh[tid >> 5][c] = s[c];
+        __syncthreads();
+        if (tid < 4) part[4 * (int64_t)blockIdx.x + tid] = (sh[0][tid] + sh[1][tid]) + (sh[2][tid] + sh[3][tid]);
+    }
+}
+
+// out[4 p + c] = sum over t < n of in[p * plane + c * comp + t * stride], over cnt; one block of
+// (4 components) x 64 threads per plane p.
+__global__ void __launch_bounds__(256) k_add_planes(const double* in, int64_t plane, int64_t comp, int64_t stride,
+                                                    int n, double cnt, double* out) {
+    const int c = threadIdx.x & 3, u = threadIdx.x >> 2;
+    double s = 0.0;
+    for (int t = u; t < n; t += 64) s += in[(int64_t)blockIdx.x * plane + c * comp + t * stride];
+    __shared__ double sh[64][4];
+    sh[u][c] = s;
+    __syncthreads();
+    if (u == 0) {
+        double a = 0.0;
+        for (int t = 0; t < 64; ++t) a += sh[t][c];
+        out[4 * blockIdx.x + c] = a / cnt;
+    }
 }
 
 // Non-equilibrium stresses xx and xy of one node, CODE/SRC/flux_X.F90:162-240
@@ -772,15 +818,16 @@ void launch_fill_xface(const Lat<S, R>& L, const Geo& g, cudaStream_t st) {
 template <typename S, typename R>
 void launch_monitor(const Lat<S, R>& L, const Geo& g, const Mask& mk, const Reduce& red, double* out,
                     cudaStream_t st) {
-    const unsigned blocks = grid_for(g.N, kTpb, (unsigned)red.max_blocks);
-    k_monitor<S, R><<<blocks, kTpb, 0, st>>>(L, g, mk, red, out);
+    const int64_t rows = (int64_t)g.m * g.n;
+    k_monitor<S, R><<<grid_for(rows, kTpb / 32, (unsigned)red.max_blocks), kTpb, 0, st>>>(L, g.l, rows, mk, red, out);
 }
 
 template <typename S, typename R>
 void launch_region_sums(const Lat<S, R>& L, const Geo& g, const Mask& mk, const uint8_t* region, const Reduce& red,
                         double* out, cudaStream_t st) {
-    const unsigned blocks = grid_for(g.N, kTpb, (unsigned)red.max_blocks);
-    k_region_sums<S, R><<<blocks, kTpb, 0, st>>>(L, g, mk, region, red, out);
+    const int64_t rows = (int64_t)g.m * g.n;
+    k_region_sums<S, R><<<grid_for(rows, kTpb / 32, (unsigned)red.max_blocks), kTpb, 0, st>>>(L, g.l, rows, mk, region,
+                                                                                             red, out);
 }
 
 template <typename S, typename R>
@@ -789,10 +836,46 @@ void launch_line(const Lat<S, R>& L, const Geo& g, int axis, int c1, int c2, dou
     k_line<S, R><<<(len + 127) / 128, 128, 0, st>>>(L, g, axis, c1, c2, out);
 }
 
+// Blocks of 128 threads: as many along x as a row fills, the rest over rows; enough shares for
+// a few waves of the 12 blocks an SM holds.
+static PlaneWalk plane_walk(const Geo& g, int axis, dim3* block, int* planes) {
+    PlaneWalk w;
+    const int tx = g.l > 64 ? 128 : (g.l > 32 ? 64 : 32);
+    *block = dim3(tx, 128 / tx);
+    *planes = axis == 0 ? 1 : (axis == 1 ? g.m : g.n);
+    w.l = g.l;
+    w.rows = axis == 0 ? g.m * g.n : (axis == 1 ? g.n : g.m);
+    w.xblocks = (g.l + tx - 1) / tx;
+    w.plane = axis == 1 ? 1 : g.m;
+    w.row = axis == 1 ? g.m : 1;
+    const int64_t most = (w.rows + (int)block->y - 1) / (int)block->y;
+    const int64_t want = 148 * 12 * (axis == 0 ? 1 : 3) / ((int64_t)*planes * w.xblocks);
+    w.shares = (int)std::max<int64_t>(1, std::min(most, want));
+    return w;
+}
+
+int64_t plane_means_scratch(const Geo& g, int axis) {
+    dim3 block;
+    int planes;
+    const PlaneWalk w = plane_walk(g, axis, &block, &planes);
+    return 4 * (axis == 0 ? (int64_t)w.shares * block.y * g.l : (int64_t)planes * w.shares * w.xblocks);
+}
+
 template <typename S, typename R>
-void launch_plane_means(const Lat<S, R>& L, const Geo& g, int axis, double* out, cudaStream_t st) {
-    const int len = axis == 0 ? g.l : (axis == 1 ? g.m : g.n);
-    k_plane_means<S, R><<<len, 256, 0, st>>>(L, g, axis, out);
+void launch_plane_means(const Lat<S, R>& L, const Geo& g, int axis, double* out, double* scratch, cudaStream_t st) {
+    dim3 block;
+    int planes;
+    const PlaneWalk w = plane_walk(g, axis, &block, &planes);
+    const unsigned blocks = (unsigned)(planes * w.shares * w.xblocks);
+    if (axis == 0) {
+        k_plane_sums<S, R, true><<<blocks, block, 0, st>>>(L, w, scratch);
+        k_add_planes<<<g.l, 256, 0, st>>>(scratch, 1, g.l, 4 * (int64_t)g.l, w.shares * (int)block.y,
+                                          (double)g.m * g.n, out);
+    } else {
+        k_plane_sums<S, R, false><<<blocks, block, 0, st>>>(L, w, scratch);
+        const int parts = w.shares * w.xblocks;
+        k_add_planes<<<planes, 256, 0, st>>>(scratch, 4 * (int64_t)parts, 1, 4, parts, (double)g.l * w.rows, out);
+    }
 }
 
 template <typename S, typename R>
@@ -843,7 +926,7 @@ void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStre
     template void launch_pack_x_rim<S, R>(const Lat<S, R>&, const Geo&, int, cudaStream_t);              \
     template void launch_unpack_x_view<S, R>(const Lat<S, R>&, const Geo&, int, const R*, cudaStream_t); \
     template void launch_line<S, R>(const Lat<S, R>&, const Geo&, int, int, int, double*, cudaStream_t);   \
-    template void launch_plane_means<S, R>(const Lat<S, R>&, const Geo&, int, double*, cudaStream_t);     \
+    template void launch_plane_means<S, R>(const Lat<S, R>&, const Geo&, int, double*, double*, cudaStream_t); \
     template void launch_cv_drag<S, R>(const Lat<S, R>&, const Geo&, const int*, R, const Reduce&, double*, \
                                        cudaStream_t);                                                     \
     template void launch_region_sums<S, R>(const Lat<S, R>&, const Geo&, const Mask&, const uint8_t*,   \
