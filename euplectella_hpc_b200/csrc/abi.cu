@@ -459,19 +459,6 @@ bool has_exchange_face(const eup_handle* h) {
     return h->cfg.bc[EUP_FRONT] == EUP_BC_EXCHANGE || h->cfg.bc[EUP_REAR] == EUP_BC_EXCHANGE;
 }
 
-// After a synchronisation: a bounded wait of the staged stream-collide kernel that ran out
-// left a step incomplete.
-int check_kernel_waits(eup_handle* h, const char* who) {
-    unsigned int n = 0;
-    CK(h, staged_wait_timeouts(&n));
-    if (n != 0)
-        return fail(h, EUP_ERR_CUDA,
-                    std::string(who) + ": " + std::to_string(n) +
-                        " bulk copies of the staged stream-collide kernel did not complete within 2 s; "
-                        "the steps since are incomplete");
-    return EUP_OK;
-}
-
 int check_handle(eup_handle* h) {
     if (!h) return fail(nullptr, EUP_ERR_INVALID_ARG, "null handle");
     cudaError_t e = cudaSetDevice(h->cfg.device);
@@ -541,8 +528,6 @@ int eup_create(const eup_config* cfg, eup_handle** out) {
     };
     cudaError_t e = cudaSetDevice(cfg->device);
     if (e != cudaSuccess) return cleanup_fail(cuda_fail(h, e, "cudaSetDevice"));
-    if ((e = prepare_stream_collide()) != cudaSuccess)
-        return cleanup_fail(cuda_fail(h, e, "stream-collide kernel attributes"));
     if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaStreamCreate"));
     const size_t lat_bytes = (size_t)Q * h->Nq * h->sbytes;
@@ -1114,7 +1099,7 @@ int eup_synchronize(eup_handle* h) {
     int rc = check_handle(h);
     if (rc) return rc;
     CK(h, cudaStreamSynchronize(h->stream));
-    return check_kernel_waits(h, "eup_synchronize");
+    return EUP_OK;
 }
 
 int eup_get_launch_count(eup_handle* h, int64_t* launches) {
@@ -1148,15 +1133,19 @@ int eup_get_force_series(eup_handle* h, int64_t first_step, int32_t count, doubl
                     "eup_get_force_series: steps " + std::to_string(first_step) + ".." +
                         std::to_string(first_step + count - 1) + " outside the recorded range " +
                         std::to_string(lo) + ".." + std::to_string(h->itime));
-    CK(h, cudaStreamSynchronize(h->stream));
-    if ((rc = check_kernel_waits(h, "eup_get_force_series"))) return rc;
-    for (int32_t c = 0; c < count;) {
+    // copies behind the steps on their stream: one wait in all for a force read every step
+    cudaError_t e = cudaSuccess;
+    for (int32_t c = 0; c < count && e == cudaSuccess;) {
         const int64_t t = first_step + c;
         const int64_t pos = t % h->cap;
         const int32_t run = (int32_t)std::min<int64_t>(count - c, h->cap - pos);
-        CK(h, cudaMemcpy(fxyz + 3 * (int64_t)c, h->series + 3 * pos, sizeof(double) * 3 * run, cudaMemcpyDeviceToHost));
+        e = cudaMemcpyAsync(fxyz + 3 * (int64_t)c, h->series + 3 * pos, sizeof(double) * 3 * run, cudaMemcpyDeviceToHost,
+                            h->stream);
         c += run;
     }
+    const cudaError_t es = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) return cuda_fail(h, e, "eup_get_force_series");
     for (int64_t t = 0; t < 3 * (int64_t)count; ++t)
         if (!std::isfinite(fxyz[t]))
             return fail(h, EUP_ERR_DIVERGED,

@@ -208,12 +208,6 @@ void launch_fill_xface(const Lat<S, R>& L, const Geo& g, cudaStream_t st);
 // planes (kStreamInterior) and the two that do (kStreamFaces), so that an x-slab can
 // receive its halo planes while the interior streams.
 enum { kStreamAll = 0, kStreamInterior = 1, kStreamFaces = 2 };
-// Kernel attributes the stream-collide launches need (once per device, outside graph capture).
-cudaError_t prepare_stream_collide();
-// Number of bounded waits of the staged stream-collide kernel that ran out on this device
-// since the last call (each stopped its CTA's stores: the step's result is then incomplete);
-// the count restarts from zero once read.
-cudaError_t staged_wait_timeouts(unsigned int* count);
 template <typename S, typename R>
 void launch_stream_collide(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g,
                            const Phys<R>& ph, int variant, cudaStream_t st, int part = kStreamAll);
