@@ -24,7 +24,7 @@ LIB_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIB_DIR, "libeup.so")
 DRIVER = os.path.join(LIB_DIR, "eup_bgk3d")
 
-SOURCES = ["abi.cu", "k_bc.cu", "halo_plan.cu", "k_step.cu", "k_setup.cu", "k_adjoint.cu", "host.cpp", "noalloc.cu"]
+SOURCES = ["abi.cu", "k_bc.cu", "halo_plan.cu", "halo_adjoint.cu", "k_step.cu", "k_setup.cu", "k_adjoint.cu", "host.cpp", "noalloc.cu"]
 HEADERS = ["lbm_common.cuh", "internal.h", "geometry.h", "halo.h", "init_eq.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC,-fopenmp,-Wall,-ffp-contract=off",

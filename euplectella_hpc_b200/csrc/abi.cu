@@ -1329,13 +1329,6 @@ struct DevBuf {
     cudaError_t alloc(size_t n) { return cudaMalloc(&p, sizeof(T) * (n > 0 ? n : 1)); }
 };
 
-template <typename T>
-cudaError_t upload_vec(DevBuf<T>& b, const std::vector<T>& v) {
-    cudaError_t e = b.alloc(v.size());
-    if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
-    return e;
-}
-
 // Lattice view of an arbitrary state buffer laid out like the handle's lattices.
 template <typename S, typename R>
 Lat<S, R> lat_at(const eup_handle* h, S* base, R* shell = nullptr) {
@@ -1514,23 +1507,13 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
     SideStream side;
     if (!serial) CK(h, side.create());
 
-    HaloAdjointTables tab;
-    std::string why;
-    if (build_halo_adjoint_tables(g, bc, &tab, &why) != EUP_OK) return fail(h, EUP_ERR_UNSUPPORTED, "eup_adjoint_run: " + why);
-    DevBuf<int64_t> d_ckey, d_cslot, d_oslot;
-    DevBuf<int32_t> d_cstart, d_ojk, d_ostart;
-    DevBuf<int8_t> d_oq;
-    CK(h, upload_vec(d_ckey, tab.copy_key));
-    CK(h, upload_vec(d_cstart, tab.copy_start));
-    CK(h, upload_vec(d_cslot, tab.copy_slot));
-    CK(h, upload_vec(d_ojk, tab.out_jk));
-    CK(h, upload_vec(d_ostart, tab.out_start));
-    CK(h, upload_vec(d_oslot, tab.out_slot));
-    CK(h, upload_vec(d_oq, tab.out_q));
     HaloAdjointDevice td;
-    td.copy_key = d_ckey.p; td.copy_start = d_cstart.p; td.copy_slot = d_cslot.p; td.ncopy = (int64_t)tab.copy_key.size();
-    td.out_jk = d_ojk.p; td.out_start = d_ostart.p; td.out_slot = d_oslot.p; td.out_q = d_oq.p;
-    td.nout = (int64_t)tab.out_jk.size();
+    std::string why;
+    const cudaError_t e_tab = build_halo_adjoint(g, bc, h->edges, &td, &why, st);
+    DevBuf<char> td_memory;
+    td_memory.p = static_cast<char*>(td.memory);
+    CK(h, e_tab);
+    if (!why.empty()) return fail(h, EUP_ERR_UNSUPPORTED, "eup_adjoint_run: " + why);
 
     // the schedule, and the states its first descent stores
     std::vector<RevAct> acts;

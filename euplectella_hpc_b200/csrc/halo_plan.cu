@@ -117,6 +117,8 @@ HaloFace record_halo_face(const Geo& g, const int bc[6], int b) {
     f.nb = z ? g.m : g.n;
     f.dst_b = x ? g.m + 2 : g.l;  // halo row stride (lbm_common.cuh, Geo::gidx)
     f.src_b = x ? g.m : (z ? (int64_t)g.l : g.lm);
+    f.lin_a = x ? g.l : 1;
+    f.lin_b = z ? (int64_t)g.l : g.lm;
     int t = 0;
     for (const Store_& s : st) {
         if (t == 5) break;
@@ -138,6 +140,7 @@ HaloFace record_halo_face(const Geo& g, const int bc[6], int b) {
         } else {
             f.kind = x ? kFaceCopyX : kFaceCopy;
             f.src_q[t] = s.v.q - 1;
+            f.lin[t] = g.lin(s.v.i, s.v.j, s.v.k);
             f.src[t] = x ? xface_idx(g, s.v.i == 1 ? 0 : 1, s.v.q - 1, 1, 1) : g.lin(s.v.i, s.v.j, s.v.k);
         }
         ++t;

@@ -132,6 +132,7 @@ struct HaloFace {
     int64_t src_b, dst_b;
     int q[5], src_q[5], da[5], db[5], lid[5];
     int64_t src[5], dst[5];
+    int64_t lin[5], lin_a, lin_b;  // interior node copied, at (0, 0), and its strides
     int pass;          // >= 0: on row b = nb-1 the old value of population `pass` goes to pass_dst + a first
     int64_t pass_dst;
 };
@@ -274,20 +275,10 @@ int64_t compact_flags(const uint8_t* flags, int64_t n, int32_t* out, void* scrat
                       cudaStream_t st, cudaError_t* err);
 
 // ---- partial bounce-back and its adjoint (k_adjoint.cu) -------------------------
-// Where the adjoint of each halo value goes, derived on the host by running the
-// reference's halo blocks on symbols.  copy_*: halo slots holding a copy of an
-// interior population, grouped by source key q*N + lin (CSR: copy_start).
-// out_*: halo slots holding an outflow equilibrium, grouped by the x = l node
-// (j-1) + (k-1)*m they are computed from, with the population produced.
-struct HaloAdjointTables {
-    std::vector<int64_t> copy_key;
-    std::vector<int32_t> copy_start;
-    std::vector<int64_t> copy_slot;
-    std::vector<int32_t> out_jk;
-    std::vector<int32_t> out_start;
-    std::vector<int64_t> out_slot;
-    std::vector<int8_t> out_q;
-};
+// Where the adjoint of each halo value goes, on the device.  copy_*: halo slots holding a copy of
+// an interior population, grouped by source key q*N + lin (CSR: copy_start), ascending within a
+// group.  out_*: halo slots holding an outflow equilibrium, grouped by the x = l node
+// (j-1) + (k-1)*m they are computed from, with the population produced, by population and slot.
 struct HaloAdjointDevice {
     const int64_t* copy_key = nullptr;
     const int32_t* copy_start = nullptr;
@@ -298,9 +289,12 @@ struct HaloAdjointDevice {
     const int64_t* out_slot = nullptr;
     const int8_t* out_q = nullptr;
     int64_t nout = 0;
+    void* memory = nullptr;  // what the arrays lie in (cudaFree)
 };
-// Returns EUP_OK or EUP_ERR_UNSUPPORTED (err says why).
-int build_halo_adjoint_tables(const Geo& g, const int bc[6], HaloAdjointTables* out, std::string* err);
+// Builds the tables from the halo plan (faces and edge table) of these flags; synchronises st.
+// cudaSuccess with *err set: the flags are not supported (err says why).
+cudaError_t build_halo_adjoint(const Geo& g, const int bc[6], const HaloEdgesDevice& edges, HaloAdjointDevice* out,
+                               std::string* err, cudaStream_t st);
 
 // One partial-bounce-back step src -> dst (any storage; FP32 arithmetic for 16-bit storage):
 // the plain stream-collide, then the mixing f* = (1 - n_s) BGK(f) + n_s f_opp on the ns_count

@@ -16,298 +16,11 @@
 //   dJ/dn_s += sum_i lambda^s_i (f_opp(i) - BGK_i(f)) + gamma_s 2 j_x
 //   lambda^{s-1}_j(x - c_j) = mu_j(x)                 (transpose of the pull)
 // plus, for populations read through the halo, the transpose of the halo
-// assignment that produced them (copies, outflow equilibria), which the host
-// derives by running the reference's halo-block sequence on symbols.
-#include <algorithm>
-#include <string>
-#include <vector>
-
-#include "../../include/eup.h"
+// assignment that produced them (copies, outflow equilibria), which
+// halo_adjoint.cu tabulates from the halo plan.
 #include "internal.h"
 
 namespace eup {
-
-// ---------------------------------------------------------------------------
-// Symbolic halo: what every halo slot holds after one step's halo blocks, as
-// a function of the state entering the step.
-// ---------------------------------------------------------------------------
-namespace {
-
-enum : int8_t { D_CONST = 0, D_COPY = 1, D_OUTFLOW = 2, D_STALE = 3 };
-struct Desc {
-    int8_t kind;
-    int8_t q;     // source population (COPY) or produced population (OUTFLOW)
-    int32_t idx;  // interior linear index (COPY) or (j-1) + (k-1)*m of x = l (OUTFLOW)
-};
-
-struct SymShell {
-    const Geo& g;
-    std::vector<Desc> d;
-    std::vector<uint8_t> pass;
-    int cur = 0;
-    explicit SymShell(const Geo& g_) : g(g_), d((size_t)Q * g_.G, Desc{D_CONST, 0, 0}), pass((size_t)Q * g_.G, 0) {}
-    size_t slot(int q, int i, int j, int k) const { return (size_t)q * g.G + (size_t)g.gidx(i, j, k); }
-    Desc ld(int q1, int i, int j, int k) const {
-        const int q = q1 - 1;
-        if (g.interior(i, j, k)) return Desc{D_COPY, (int8_t)q, (int32_t)g.lin(i, j, k)};
-        const size_t s = slot(q, i, j, k);
-        Desc v = d[s];
-        // written in the previous step and not yet in this one: a value of an older state
-        if (cur == 2 && pass[s] == 1 && v.kind != D_CONST) v.kind = D_STALE;
-        return v;
-    }
-    void st(int q1, int i, int j, int k, Desc v) {
-        const size_t s = slot(q1 - 1, i, j, k);
-        d[s] = v;
-        pass[s] = (uint8_t)cur;
-    }
-};
-
-// The halo blocks of CODE/SRC/bcond.bc.F90 in the reference's order, on
-// symbols; the same ranges and assignments as the kernels of k_bc.cu.
-void sym_halo_step(SymShell& S, const int bc[6]) {
-    const Geo& g = S.g;
-    const int l = g.l, m = g.m, n = g.n, l1 = l + 1, m1 = m + 1, n1 = n + 1;
-    const Desc cst{D_CONST, 0, 0};
-    auto LD = [&](int q, int i, int j, int k) { return S.ld(q, i, j, k); };
-    auto ST = [&](int q, int i, int j, int k, Desc v) { S.st(q, i, j, k, v); };
-    // front
-    if (bc[0] == 0) {
-        for (int k = 1; k <= n; ++k) {
-            ST(12, l1, 0, k, LD(12, 1, m, k));
-            for (int j = 1; j <= m; ++j)
-                for (int q = 10; q <= 14; ++q) ST(q, l1, j, k, LD(q, 1, j, k));
-        }
-    } else if (bc[0] == 1) {
-        for (int k = 1; k <= n; ++k)
-            for (int j = 1; j <= m; ++j) {
-                const Desc v1 = LD(1, l, j, k), v2 = LD(2, l, j, k), v3 = LD(3, l, j, k), v4 = LD(4, l, j, k),
-                           v5 = LD(5, l, j, k);
-                ST(12, l1, j - 1, k, v1);
-                ST(13, l1, j, k - 1, v2);
-                ST(10, l1, j + 1, k, v3);
-                ST(11, l1, j, k + 1, v4);
-                ST(14, l1, j, k, v5);
-            }
-    } else {
-        for (int k = 1; k <= n; ++k)
-            for (int j = 1; j <= m; ++j)
-                for (int q = 10; q <= 14; ++q) ST(q, l1, j, k, Desc{D_OUTFLOW, (int8_t)(q - 1), (j - 1) + (k - 1) * m});
-        for (int j = 1; j <= m; ++j)
-            for (int q = 10; q <= 14; ++q) {
-                const Desc lo = LD(q, l1, j, 1), hi = LD(q, l1, j, n);
-                ST(q, l1, j, 0, lo);
-                ST(q, l1, j, n1, hi);
-            }
-        for (int k = 1; k <= n; ++k)
-            for (int q = 10; q <= 14; ++q) {
-                const Desc lo = LD(q, l1, 1, k), hi = LD(q, l1, m, k);
-                ST(q, l1, 0, k, lo);
-                ST(q, l1, m1, k, hi);
-            }
-    }
-    // rear
-    if (bc[1] == 0) {
-        for (int k = 1; k <= n; ++k) {
-            ST(1, 0, m1, k, LD(1, l, 1, k));
-            for (int j = 1; j <= m; ++j)
-                for (int q = 1; q <= 5; ++q) ST(q, 0, j, k, LD(q, l, j, k));
-        }
-    } else if (bc[1] == 1) {
-        for (int k = 1; k <= n; ++k)
-            for (int j = 1; j <= m; ++j) {
-                const Desc v10 = LD(10, 1, j, k), v11 = LD(11, 1, j, k), v12 = LD(12, 1, j, k),
-                           v13 = LD(13, 1, j, k), v14 = LD(14, 1, j, k);
-                ST(3, 0, j - 1, k, v10);
-                ST(4, 0, j, k - 1, v11);
-                ST(1, 0, j + 1, k, v12);
-                ST(2, 0, j, k + 1, v13);
-                ST(5, 0, j, k, v14);
-            }
-    } else {
-        for (int k = 0; k <= n1; ++k)
-            for (int j = 0; j <= m1; ++j)
-                for (int q = 1; q <= 5; ++q) ST(q, 0, j, k, cst);
-    }
-    // up
-    if (bc[4] == 0) {
-        for (int j = 1; j <= m; ++j)
-            for (int i = 1; i <= l; ++i) {
-                const int qs[5] = {2, 9, 11, 15, 16};
-                for (int q : qs) ST(q, i, j, n1, LD(q, i, j, 1));
-            }
-    } else if (bc[4] == 1 || bc[4] == 2) {
-        for (int j = 1; j <= m; ++j)
-            for (int i = 1; i <= l; ++i) {
-                const Desc v6 = LD(6, i, j, n), v13 = LD(13, i, j, n), v18 = LD(18, i, j, n), v4 = LD(4, i, j, n),
-                           v7 = LD(7, i, j, n);
-                ST(15, i, j, n1, v6);
-                ST(2, i - 1, j, n1, v13);
-                ST(9, i, j - 1, n1, v18);
-                ST(11, i + 1, j, n1, v4);
-                ST(16, i, j + 1, n1, v7);
-            }
-    } else {
-        for (int j = 0; j <= m1; ++j)
-            for (int i = 0; i <= l1; ++i) {
-                const Desc v6 = LD(6, i, j, n), v13 = LD(13, i, j, n), v18 = LD(18, i, j, n), v4 = LD(4, i, j, n),
-                           v7 = LD(7, i, j, n);
-                ST(15, i, j, n1, v6);
-                ST(11, i, j, n1, v13);
-                ST(16, i, j, n1, v18);
-                ST(2, i, j, n1, v4);
-                ST(9, i, j, n1, v7);
-            }
-    }
-    // down
-    for (int j = 1; j <= m; ++j)
-        for (int i = 1; i <= l; ++i) {
-            if (bc[5] == 0) {
-                const int qs[5] = {4, 6, 7, 13, 18};
-                for (int q : qs) ST(q, i, j, 0, LD(q, i, j, n));
-            } else if (bc[5] == 1) {
-                const Desc v15 = LD(15, i, j, 1), v11 = LD(11, i, j, 1), v16 = LD(16, i, j, 1), v2 = LD(2, i, j, 1),
-                           v9 = LD(9, i, j, 1);
-                ST(6, i, j, 0, v15);
-                ST(4, i - 1, j, 0, v11);
-                ST(7, i, j - 1, 0, v16);
-                ST(13, i + 1, j, 0, v2);
-                ST(18, i, j + 1, 0, v9);
-            } else {
-                const Desc v15 = LD(15, i, j, 1), v11 = LD(11, i, j, 1), v16 = LD(16, i, j, 1), v2 = LD(2, i, j, 1),
-                           v9 = LD(9, i, j, 1);
-                ST(6, i, j, 0, v15);
-                ST(13, i, j, 0, v11);
-                ST(18, i, j, 0, v16);
-                ST(4, i, j, 0, v2);
-                ST(7, i, j, 0, v9);
-            }
-        }
-    // left
-    for (int k = 1; k <= n; ++k) {
-        if (bc[3] == 0) ST(3, 0, 0, k, LD(3, l, m, k));
-        for (int i = 1; i <= l; ++i) {
-            if (bc[3] == 0) {
-                const int qs[5] = {3, 7, 8, 9, 12};
-                Desc v[5];
-                for (int t = 0; t < 5; ++t) v[t] = LD(qs[t], i, m, k);
-                for (int t = 0; t < 5; ++t) ST(qs[t], i, 0, k, v[t]);
-            } else if (bc[3] == 1) {
-                const Desc v17 = LD(17, i, 1, k), v1 = LD(1, i, 1, k), v10 = LD(10, i, 1, k), v16 = LD(16, i, 1, k),
-                           v18 = LD(18, i, 1, k);
-                ST(8, i, 0, k, v17);
-                ST(12, i + 1, 0, k, v1);
-                ST(3, i - 1, 0, k, v10);
-                ST(7, i, 0, k - 1, v16);
-                ST(9, i, 0, k + 1, v18);
-            } else {
-                const Desc v17 = LD(17, i, 1, k), v1 = LD(1, i, 1, k), v10 = LD(10, i, 1, k), v16 = LD(16, i, 1, k),
-                           v18 = LD(18, i, 1, k);
-                ST(8, i, 0, k, v17);
-                ST(3, i, 0, k, v1);
-                ST(12, i, 0, k, v10);
-                ST(9, i, 0, k, v16);
-                ST(7, i, 0, k, v18);
-            }
-        }
-    }
-    // right
-    for (int k = 1; k <= n; ++k) {
-        if (bc[2] == 0) ST(10, l1, m1, k, LD(10, 1, 1, k));
-        for (int i = 1; i <= l; ++i) {
-            if (bc[2] == 0) {
-                const int qs[5] = {1, 10, 16, 17, 18};
-                Desc v[5];
-                for (int t = 0; t < 5; ++t) v[t] = LD(qs[t], i, 1, k);
-                for (int t = 0; t < 5; ++t) ST(qs[t], i, m1, k, v[t]);
-            } else if (bc[2] == 1) {
-                const Desc v3 = LD(3, i, m, k), v7 = LD(7, i, m, k), v8 = LD(8, i, m, k), v9 = LD(9, i, m, k),
-                           v12 = LD(12, i, m, k);
-                ST(10, i + 1, m1, k, v3);
-                ST(16, i, m1, k + 1, v7);
-                ST(17, i, m1, k, v8);
-                ST(18, i, m1, k - 1, v9);
-                ST(1, i - 1, m1, k, v12);
-            } else {
-                const Desc v3 = LD(3, i, m, k), v7 = LD(7, i, m, k), v8 = LD(8, i, m, k), v9 = LD(9, i, m, k),
-                           v12 = LD(12, i, m, k);
-                ST(1, i, m1, k, v3);
-                ST(18, i, m1, k, v7);
-                ST(17, i, m1, k, v8);
-                ST(16, i, m1, k, v9);
-                ST(10, i, m1, k, v12);
-            }
-        }
-    }
-    // free-slip edge fixes
-    for (int i = 1; i <= l; ++i) {
-        if (bc[3] == 3 && bc[4] == 3) ST(9, i, 0, n1, LD(18, i, 1, n));
-        if (bc[2] == 3 && bc[4] == 3) ST(16, i, m1, n1, LD(7, i, m, n));
-        if (bc[2] == 3 && bc[5] == 3) ST(18, i, m1, 0, LD(9, i, m, 1));
-        if (bc[3] == 3 && bc[5] == 3) ST(7, i, 0, 0, LD(16, i, 1, 1));
-    }
-}
-
-}  // namespace
-
-int build_halo_adjoint_tables(const Geo& g, const int bc[6], HaloAdjointTables* out, std::string* err) {
-    SymShell S(g);
-    S.cur = 1;
-    sym_halo_step(S, bc);
-    S.cur = 2;
-    sym_halo_step(S, bc);
-    out->copy_key.clear();
-    out->copy_start.clear();
-    out->copy_slot.clear();
-    out->out_jk.clear();
-    out->out_start.clear();
-    out->out_slot.clear();
-    out->out_q.clear();
-    struct CE { int64_t key; int64_t slot; };
-    struct OE { int32_t jk; int64_t slot; int8_t q; };
-    std::vector<CE> ce;
-    std::vector<OE> oe;
-    // pulled halo slots: (q, h) with h + c_q interior
-    for (int q = 0; q < 18; ++q) {
-        for (int k = 0; k <= g.n + 1; ++k)
-            for (int j = 0; j <= g.m + 1; ++j)
-                for (int i = 0; i <= g.l + 1; ++i) {
-                    if (g.interior(i, j, k)) continue;
-                    if (!g.interior(i + cx_of(q), j + cy_of(q), k + cz_of(q))) continue;
-                    const size_t s = S.slot(q, i, j, k);
-                    const Desc d = S.d[s];
-                    if (d.kind == D_STALE) {
-                        *err = "the adjoint needs every halo value of a step to follow from the state entering it; "
-                               "with these boundary flags a halo block reads a value written one step earlier";
-                        return EUP_ERR_UNSUPPORTED;
-                    }
-                    if (d.kind == D_COPY) ce.push_back(CE{(int64_t)d.q * g.N + d.idx, (int64_t)s});
-                    if (d.kind == D_OUTFLOW) oe.push_back(OE{d.idx, (int64_t)s, d.q});
-                }
-    }
-    std::sort(ce.begin(), ce.end(), [](const CE& a, const CE& b) { return a.key < b.key || (a.key == b.key && a.slot < b.slot); });
-    for (size_t t = 0; t < ce.size(); ++t) {
-        if (t == 0 || ce[t].key != ce[t - 1].key) {
-            out->copy_key.push_back(ce[t].key);
-            out->copy_start.push_back((int32_t)t);
-        }
-        out->copy_slot.push_back(ce[t].slot);
-    }
-    out->copy_start.push_back((int32_t)ce.size());
-    std::sort(oe.begin(), oe.end(), [](const OE& a, const OE& b) {
-        return a.jk < b.jk || (a.jk == b.jk && (a.q < b.q || (a.q == b.q && a.slot < b.slot)));
-    });
-    for (size_t t = 0; t < oe.size(); ++t) {
-        if (t == 0 || oe[t].jk != oe[t - 1].jk) {
-            out->out_jk.push_back(oe[t].jk);
-            out->out_start.push_back((int32_t)t);
-        }
-        out->out_slot.push_back(oe[t].slot);
-        out->out_q.push_back(oe[t].q);
-    }
-    out->out_start.push_back((int32_t)oe.size());
-    return EUP_OK;
-}
 
 // ---------------------------------------------------------------------------
 // Kernels

@@ -176,6 +176,25 @@ struct Geo {
         if (k == 0) return oz0 + (int64_t)(j - 1) * l + (i - 1);
         return ozn + (int64_t)(j - 1) * l + (i - 1);
     }
+    // the halo node of shell index s (the inverse of gidx)
+    __host__ __device__ __forceinline__ void shell_node(int64_t s, int* i, int* j, int* k) const {
+        if (s < oy0) {
+            *i = s < oxl ? 0 : l + 1;
+            const int64_t r = s < oxl ? s : s - oxl;
+            *j = (int)(r % (m + 2));
+            *k = (int)(r / (m + 2));
+        } else if (s < oz0) {
+            *j = s < oym ? 0 : m + 1;
+            const int64_t r = s - (s < oym ? oy0 : oym);
+            *i = (int)(r % l) + 1;
+            *k = (int)(r / l);
+        } else {
+            *k = s < ozn ? 0 : n + 1;
+            const int64_t r = s - (s < ozn ? oz0 : ozn);
+            *i = (int)(r % l) + 1;
+            *j = (int)(r / l) + 1;
+        }
+    }
 };
 
 // Row (j, k) of face row index f, 0 <= f < nz m + (n-2) ny (nz = 2 for n >= 2, else 1;
