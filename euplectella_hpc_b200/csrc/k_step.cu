@@ -7,6 +7,8 @@
 // through the halo shell.
 #include <string.h>
 
+#include <type_traits>
+
 #include "internal.h"
 
 namespace eup {
@@ -146,13 +148,19 @@ __device__ __forceinline__ void node_step(const Lat<S, R>& src, const Lat<S, R>&
     scatter_node(dst, g, i, j, k, rowlin, x);
 }
 
+// Plane of thread block z: upwards, or with DOWN from k = n down (see launch_stream_collide).
+template <bool DOWN>
+__device__ __forceinline__ int plane_of_block(const Geo& g) {
+    return DOWN ? g.n - (int)blockIdx.z : (int)blockIdx.z + 1;
+}
+
 // One thread per node of the columns i0 .. i0+ni-1; grid (ceil(ni/bx), m, n).
-template <typename S, typename R>
+template <typename S, typename R, bool DOWN>
 __global__ void __launch_bounds__(128) k_stream_collide_scalar(Lat<S, R> src, Lat<S, R> dst, Geo g, Phys<R> ph,
                                                                int i0, int ni) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ni) return;
-    node_step(src, dst, g, ph, i0 + t, (int)blockIdx.y + 1, (int)blockIdx.z + 1);
+    node_step(src, dst, g, ph, i0 + t, (int)blockIdx.y + 1, plane_of_block<DOWN>(g));
 }
 
 // The columns i = 1 and i = l (the only ones that pull from the x halo planes): one thread
@@ -221,40 +229,60 @@ __device__ __forceinline__ void load_pair_raw(const PullBase<S>& pb, int i, int 
     for (int q = 0; q < 19; ++q) r[q] = *reinterpret_cast<const T2*>(pb.p[q] + x);
 }
 
+// The x-halo values of the first (LO: node i = 1 in the low lane) and last (HI: node i+1 = l in
+// the high lane) node of a row replace what the shifted loads brought.
+template <typename S>
+__device__ __forceinline__ void x_halo_ends(const Lat<S, float>& src, const Geo& g, bool lo, bool hi, int j, int k,
+                                            F2 (&x)[19]) {
+    using K = KOps<S, float>;
+    if (lo) {
+#pragma unroll
+        for (int q = 0; q < 18; ++q)
+            if (cx_of(q) == 1)
+                x[q].v.x = K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(0, j - cy_of(q), k - cz_of(q))], q, src);
+    }
+    if (hi) {
+#pragma unroll
+        for (int q = 0; q < 18; ++q)
+            if (cx_of(q) == -1)
+                x[q].v.y =
+                    K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(g.l + 1, j - cy_of(q), k - cz_of(q))], q, src);
+    }
+}
+
+// x-face copy of the first/last column: the value a later load returns.
+template <typename S>
+__device__ __forceinline__ void store_x_face(const Lat<S, float>& dst, const Geo& g, bool lo, bool hi, int j, int k,
+                                             const F2 (&x)[19]) {
+    using V2 = Vec2<S>;
+    if (lo | hi) {
+#pragma unroll
+        for (int q = 0; q < 18; ++q) {
+            const typename V2::T o = V2::pack(x[q].v);
+            if (lo) dst.xface[xface_idx(g, 0, q, j, k)] = Store<S, float>::load(V2::lo(o), q, dst.inv_scale);
+            if (hi) dst.xface[xface_idx(g, 1, q, j, k)] = Store<S, float>::load(V2::hi(o), q, dst.inv_scale);
+        }
+    }
+}
+
+template <typename S>
+__device__ __forceinline__ void collide_pair(const Lat<S, float>& src, const Phys<float>& ph, F2 (&x)[19]) {
+    if constexpr (DevStore<S>::value) collide_dev<F2>(x, ph.omega, ph.omega1, ph.fgrad, src.scale, src.inv_scale);
+    else collide<F2>(x, F2(ph.omega), F2(ph.omega1), F2(ph.fgrad));
+}
+
 // Everything after the pulls of a pair: the x-halo values of the first and
 // last node of the row, the collision of both nodes as packed FP32, the x-face copy and
 // the stores.
 template <typename S>
 __device__ __forceinline__ void finish_pair(const Lat<S, float>& src, const Lat<S, float>& dst, const Geo& g,
                                             const Phys<float>& ph, int i, int j, int k, int rowlin, F2 (&x)[19]) {
-    using K = KOps<S, float>;
     using V2 = Vec2<S>;
     using T2 = typename V2::T;
     constexpr bool dev = DevStore<S>::value;
-    const int l = g.l;
-    if (i == 1) {
-#pragma unroll
-        for (int q = 0; q < 18; ++q)
-            if (cx_of(q) == 1)
-                x[q].v.x = K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(0, j - cy_of(q), k - cz_of(q))], q, src);
-    }
-    if (i + 1 == l) {
-#pragma unroll
-        for (int q = 0; q < 18; ++q)
-            if (cx_of(q) == -1)
-                x[q].v.y =
-                    K::from_shell(src.ghost[(int64_t)q * g.G + g.gidx(l + 1, j - cy_of(q), k - cz_of(q))], q, src);
-    }
-    if constexpr (dev) collide_dev<F2>(x, ph.omega, ph.omega1, ph.fgrad, src.scale, src.inv_scale);
-    else collide<F2>(x, F2(ph.omega), F2(ph.omega1), F2(ph.fgrad));
-    if ((i == 1) | (i + 1 == l)) {  // x-face copy of the first/last column: the value a later load returns
-#pragma unroll
-        for (int q = 0; q < 18; ++q) {
-            const T2 o = V2::pack(x[q].v);
-            if (i == 1) dst.xface[xface_idx(g, 0, q, j, k)] = Store<S, float>::load(V2::lo(o), q, dst.inv_scale);
-            if (i + 1 == l) dst.xface[xface_idx(g, 1, q, j, k)] = Store<S, float>::load(V2::hi(o), q, dst.inv_scale);
-        }
-    }
+    x_halo_ends(src, g, i == 1, i + 1 == g.l, j, k, x);
+    collide_pair<S>(src, ph, x);
+    store_x_face<S>(dst, g, i == 1, i + 1 == g.l, j, k, x);
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
         const T2 o = V2::pack(x[q].v);
@@ -356,12 +384,12 @@ __device__ __forceinline__ void pair_step(const Lat<S, float>& src, const Lat<S,
 }
 
 // Pairs p0 .. p0+np-1 of every row (pair p: nodes 2p+1, 2p+2); grid (ceil(np/128), m, n).
-template <typename S, int MINB>
+template <typename S, int MINB, bool DOWN>
 __global__ void __launch_bounds__(128, MINB) k_stream_collide_pair(Lat<S, float> src, Lat<S, float> dst, Geo g,
                                                                    Phys<float> ph, PullBase<S> pb, int p0, int np) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (t >= np) return;
-    pair_step(src, dst, g, ph, pb, 2 * (p0 + t) + 1, (int)blockIdx.y + 1, (int)blockIdx.z + 1);
+    pair_step(src, dst, g, ph, pb, 2 * (p0 + t) + 1, (int)blockIdx.y + 1, plane_of_block<DOWN>(g));
 }
 
 // The first and last pair of every row (the only ones that pull from the x halo planes):
@@ -374,6 +402,20 @@ __global__ void __launch_bounds__(128, 6) k_stream_collide_pair_faces(Lat<S, flo
     const int side = (int)(t % sides);
     const int64_t row = t / sides;
     pair_step(src, dst, g, ph, pb, side ? g.l - 1 : 1, (int)(row % g.m) + 1, (int)(row / g.m) + 1);
+}
+
+// Whether a step walks the planes from k = n down.  A step leaves the planes it wrote last in
+// L2 (126 MB), and a step that starts with them finds them there: successive steps walk in
+// turn, since they swap source and destination and the direction is the order of the two in
+// memory.  Step with all upward / in turn: 256x128x64 FP32 (159 MB a lattice) 68.1 / 64.7 us, FP16
+// 53.4 / 48.8, FP64 118.4 / 116.3; 127^3 FP32 75.6 / 70.8; 384x192x192 FP32 (1.1 GB) 358.9 / 354.6,
+// FP16 242 / 234.  At 768x384x384 FP32 (8.6 GB) nothing is left of it, and the downward 16-bit
+// kernel, whose plane index takes one more register, was the slower by 2 % there: beyond 2 GB
+// every step goes up.
+template <typename S, typename R>
+bool sweep_down(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g) {
+    if ((double)g.N * Q * sizeof(S) > 2147483648.0) return false;
+    return reinterpret_cast<uintptr_t>(src.pop[0]) > reinterpret_cast<uintptr_t>(dst.pop[0]);
 }
 
 template <typename S, typename R>
@@ -417,13 +459,18 @@ bool launch_pair(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const
         // resident blocks of 128 threads per SM the register budget is sized for: by default
         // 6 (80 registers) for FP32 storage, 8 (64) for 16-bit storage, whose loads need fewer
         const int minb = occ > 0 ? occ + 3 : (sizeof(S) == 4 ? 6 : 8);
-        switch (minb) {
-            case 4: k_stream_collide_pair<S, 4><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-            case 5: k_stream_collide_pair<S, 5><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-            case 6: k_stream_collide_pair<S, 6><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-            case 7: k_stream_collide_pair<S, 7><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-            default: k_stream_collide_pair<S, 8><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-        }
+        auto launch = [&](auto down) {
+            constexpr bool D = decltype(down)::value;
+            switch (minb) {
+                case 4: k_stream_collide_pair<S, 4, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
+                case 5: k_stream_collide_pair<S, 5, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
+                case 6: k_stream_collide_pair<S, 6, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
+                case 7: k_stream_collide_pair<S, 7, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
+                default: k_stream_collide_pair<S, 8, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
+            }
+        };
+        if (sweep_down(src, dst, g)) launch(std::true_type());
+        else launch(std::false_type());
         return true;
     }
 }
@@ -596,7 +643,8 @@ void launch_stream_collide(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo
     const int ni = part == kStreamInterior ? g.l - 2 : g.l;
     if (ni <= 0) return;
     dim3 grid((ni + bx - 1) / bx, g.m, g.n);
-    k_stream_collide_scalar<S, R><<<grid, bx, 0, st>>>(src, dst, g, ph, i0, ni);
+    if (sweep_down(src, dst, g)) k_stream_collide_scalar<S, R, true><<<grid, bx, 0, st>>>(src, dst, g, ph, i0, ni);
+    else k_stream_collide_scalar<S, R, false><<<grid, bx, 0, st>>>(src, dst, g, ph, i0, ni);
 }
 
 template void launch_stream_collide<float, float>(const Lat<float, float>&, const Lat<float, float>&,
