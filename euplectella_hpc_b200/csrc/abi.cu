@@ -16,6 +16,10 @@
 
 using namespace eup;
 
+// Steps per graph of a long run (even: a run ends on the lattice it started from), and the run
+// length from which such a graph is made.
+constexpr int kChunkSteps = 16, kChunkFrom = 32;
+
 struct eup_handle {
     eup_config cfg{};
     Geo g{};
@@ -29,6 +33,7 @@ struct eup_handle {
     HaloEdgesDevice edges;        // stores of the halo's edge lines (edges.e owned by the handle)
     int64_t* d_itime = nullptr;   // device copy of the step counter (series slot of the drag)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one time step, source lattice 0 or 1
+    cudaGraphExec_t chunk[2] = {nullptr, nullptr};  // kChunkSteps of them, starting from lattice 0 or 1
     int cur = 0;
     uint32_t* bits = nullptr;
     int wpr = 0;
@@ -163,7 +168,8 @@ struct PhaseEvents {
 // step counter), halo planes in the reference's order, stream-collide.
 // Returns the number of kernels launched.
 template <typename S, typename R>
-int enqueue_one_step(eup_handle* h, int src_idx, PhaseEvents* pe, size_t s) {
+int enqueue_one_step(eup_handle* h, int src_idx, PhaseEvents* pe, size_t s, bool chained = false) {
+    const LaunchTo to(h->stream, chained);
     const Phys<R> ph = make_phys<R>(h);
     const int bc[6] = {h->cfg.bc[0], h->cfg.bc[1], h->cfg.bc[2], h->cfg.bc[3], h->cfg.bc[4], h->cfg.bc[5]};
     const Lat<S, R> src = make_lat<S, R>(h, src_idx), dst = make_lat<S, R>(h, src_idx ^ 1);
@@ -171,22 +177,22 @@ int enqueue_one_step(eup_handle* h, int src_idx, PhaseEvents* pe, size_t s) {
     if (pe) pe->mark(4 * s + 0, h->stream);
     if (h->pbb) {  // partial bounce-back: halo planes, stream-collide, mixing and force of the step
         if (pe) pe->mark(4 * s + 1, h->stream);
-        n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h));
+        n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, to, bc_separate(h));
         if (pe) pe->mark(4 * s + 2, h->stream);
         launch_pbb_step<S, R>(src, dst, h->g, ph, static_cast<const R*>(h->ns), h->ns_list, h->ns_count,
-                              make_reduce(h), h->series, h->cap, h->d_itime, h->stream);
+                              make_reduce(h), h->series, h->cap, h->d_itime, to);
         if (pe) pe->mark(4 * s + 3, h->stream);
         return n + 2;
     }
     // boundaries: bounce-back then halo planes (CODE/SRC/boundaries.F90:36-49,235-248)
     const ForceSum force = launch_bounce<S, R>(src, h->g, h->links, make_reduce(h), h->series, h->cap, h->d_itime,
-                                               h->stream);
+                                               to);
     n += force.blocks > 0;
     if (pe) pe->mark(4 * s + 1, h->stream);
-    n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, h->stream, bc_separate(h), &force);
+    n += launch_bc<S, R>(src, h->g, bc, ph, h->edges, to, bc_separate(h), &force);
     if (pe) pe->mark(4 * s + 2, h->stream);
     // propagation + collision (CODE/SRC/bgk3d.F90:133-138)
-    launch_stream_collide<S, R>(src, dst, h->g, ph, h->variant, h->stream);
+    launch_stream_collide<S, R>(src, dst, h->g, ph, h->variant, to);
     n += 1;
     if (pe) pe->mark(4 * s + 3, h->stream);
     return n;
@@ -243,28 +249,35 @@ void unpack_x_view_dispatch(eup_handle* h, int side, const void* src) {
     h->launches += 1;
 }
 
+// Captures `steps` steps from lattice p into *exec, their kernels chained.
+template <typename S, typename R>
+cudaError_t capture_steps(eup_handle* h, int p, int steps, cudaGraphExec_t* exec, int* per_step) {
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    for (int s = 0; s < steps; ++s) *per_step = enqueue_one_step<S, R>(h, p ^ (s & 1), nullptr, 0, true);
+    e = cudaStreamEndCapture(h->stream, &graph);
+    if (e != cudaSuccess) return e;
+    e = cudaGraphInstantiate(exec, graph, 0);
+    cudaGraphDestroy(graph);
+    return e;
+}
+
 template <typename S, typename R>
 cudaError_t capture_graphs(eup_handle* h, int* per_step) {
     for (int p = 0; p < 2; ++p) {
         if (h->graph[p]) continue;
-        cudaGraph_t graph = nullptr;
-        cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return e;
-        *per_step = enqueue_one_step<S, R>(h, p, nullptr, 0);
-        e = cudaStreamEndCapture(h->stream, &graph);
-        if (e != cudaSuccess) return e;
-        e = cudaGraphInstantiate(&h->graph[p], graph, 0);
-        cudaGraphDestroy(graph);
+        const cudaError_t e = capture_steps<S, R>(h, p, 1, &h->graph[p], per_step);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
 void drop_graphs(eup_handle* h) {
-    for (auto& g : h->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
+    for (cudaGraphExec_t* g : {&h->graph[0], &h->graph[1], &h->chunk[0], &h->chunk[1]})
+        if (*g) {
+            cudaGraphExecDestroy(*g);
+            *g = nullptr;
         }
 }
 
@@ -282,7 +295,21 @@ cudaError_t enqueue_steps(eup_handle* h, int32_t nsteps, PhaseEvents* pe = nullp
         if (e != cudaSuccess) return e;
         if (per_step == 0) per_step = h->launches_per_step;
         h->launches_per_step = per_step;
-        for (int32_t s = 0; s < nsteps; ++s) {
+        int32_t s = 0;
+        if (nsteps >= kChunkFrom) {
+            // runs of steps as one graph each, from the lattice the run starts with
+            if (!h->chunk[h->cur]) {
+                e = capture_steps<S, R>(h, h->cur, kChunkSteps, &h->chunk[h->cur], &per_step);
+                if (e != cudaSuccess) return e;
+            }
+            for (; s + kChunkSteps <= nsteps; s += kChunkSteps) {
+                e = cudaGraphLaunch(h->chunk[h->cur], h->stream);
+                if (e != cudaSuccess) return e;
+                h->launches += (int64_t)per_step * kChunkSteps;
+                h->itime += kChunkSteps;
+            }
+        }
+        for (; s < nsteps; ++s) {
             e = cudaGraphLaunch(h->graph[h->cur], h->stream);
             if (e != cudaSuccess) return e;
             h->launches += per_step;

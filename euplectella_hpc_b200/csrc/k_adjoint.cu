@@ -82,6 +82,7 @@ template <typename S, typename R>
 __global__ void __launch_bounds__(256) k_pbb_list(Lat<S, R> src, Lat<S, R> dst, Geo g, const R* ns,
                                                   const int32_t* list, int64_t nlist, Reduce red, double* series,
                                                   int64_t cap, int64_t* d_itime) {
+    chain_begin();
     using P = PState<S, R>;
     double f[3] = {0.0, 0.0, 0.0};
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nlist;
@@ -356,10 +357,10 @@ unsigned capped_grid(int64_t work, int tpb) {
 template <typename S, typename R>
 void launch_pbb_step(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph, const R* ns,
                      const int32_t* ns_list, int64_t ns_count, const Reduce& red, double* series, int64_t cap,
-                     int64_t* d_itime, cudaStream_t st) {
-    launch_stream_collide<S, R>(src, dst, g, ph, 0, st);
-    k_pbb_list<S, R><<<capped_grid(ns_count, 256), 256, 0, st>>>(src, dst, g, ns, ns_list, ns_count, red, series,
-                                                                  cap, d_itime);
+                     int64_t* d_itime, const LaunchTo& to) {
+    launch_stream_collide<S, R>(src, dst, g, ph, 0, to);
+    launch(k_pbb_list<S, R>, capped_grid(ns_count, 256), 256, to, src, dst, g, ns, ns_list, ns_count, red, series, cap,
+           d_itime);
 }
 
 template <typename S, typename R>
@@ -394,7 +395,7 @@ void launch_pbb_adjoint(const Lat<S, R>& f, const Geo& g, const Phys<R>& ph, con
 #define EUP_PBB_INST(S, R)                                                                                       \
     template void launch_pbb_step<S, R>(const Lat<S, R>&, const Lat<S, R>&, const Geo&, const Phys<R>&, const R*, \
                                         const int32_t*, int64_t, const Reduce&, double*, int64_t, int64_t*,        \
-                                        cudaStream_t);                                                             \
+                                        const LaunchTo&);                                                             \
     template void launch_pbb_adjoint<S, R>(const Lat<S, R>&, const Geo&, const Phys<R>&, const R*,                \
                                            const Lat<R, R>&, const Lat<R, R>&, R*, double*, R,                     \
                                            const HaloAdjointDevice&, cudaStream_t, int);

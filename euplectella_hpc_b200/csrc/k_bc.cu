@@ -87,6 +87,7 @@ __device__ __forceinline__ void sum_partials(const ForceSum& a, bool advance) {
 
 template <typename S, typename R>
 __global__ void __launch_bounds__(kTpb) k_bounce(const __grid_constant__ BounceArgs<S, R> p) {
+    chain_begin();
     double f[3] = {0.0, 0.0, 0.0};
     const int64_t total = p.links.nfluid + p.links.nhalo;
     for (int64_t t = (int64_t)blockIdx.x * kTpb + threadIdx.x; t < total; t += (int64_t)gridDim.x * kTpb) {
@@ -202,6 +203,7 @@ __device__ __forceinline__ void outflow_row(const Lat<S, R>& L, const Geo& g, in
 
 template <typename S, typename R>
 __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<S, R> p) {
+    chain_begin();
     int s = 0;
 #pragma unroll
     for (int i = 1; i < kHaloSegments; ++i) s += blockIdx.x >= p.first[i];
@@ -699,18 +701,18 @@ void launch_unpack_x(const Lat<S, R>& L, const Geo& g, int side, const R* in, cu
 
 template <typename S, typename R>
 int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& ph, const HaloEdgesDevice& edges,
-              cudaStream_t st, bool separate, const ForceSum* force) {
+              const LaunchTo& to, bool separate, const ForceSum* force) {
     HaloPlan<S, R> p{};
     p.L = L;
     p.g = g;
     p.force = ph.force;
     halo_inflow(ph.u_inflow, p.inflow);
     int n = 0, launches = 0;
-    auto launch = [&] {
+    auto run = [&] {
         if (n == 0) return;
         const unsigned blocks = p.first[n];
         for (int s = n; s <= kHaloSegments; ++s) p.first[s] = 0xffffffffu;  // no block reaches them
-        k_halo<S, R><<<blocks, kTpb, 0, st>>>(p);
+        launch(k_halo<S, R>, blocks, kTpb, to, p);
         ++launches;
         n = 0;
         p.first[0] = 0;
@@ -763,9 +765,9 @@ int launch_bc(const Lat<S, R>& L, const Geo& g, const int bc[6], const Phys<R>& 
             f.edges = edges.e + edges.first[b];
             add(f);
         }
-        if (separate && n > before) launch();
+        if (separate && n > before) run();
     }
-    launch();
+    run();
     return launches;
 }
 
@@ -789,13 +791,13 @@ BounceArgs<S, R> bounce_args(const Lat<S, R>& L, const Geo& g, const LinksDevice
 
 template <typename S, typename R>
 ForceSum launch_bounce(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
-                       int64_t cap, int64_t* d_itime, cudaStream_t st) {
+                       int64_t cap, int64_t* d_itime, const LaunchTo& to) {
     ForceSum sum{red.partials, 0, series, cap, d_itime};
     if (links.nfluid + links.nhalo == 0) return sum;
     BounceArgs<S, R> p = bounce_args(L, g, links, red);
     p.bounce = 1;
     sum.blocks = (int)grid_for(links.nfluid + links.nhalo, kTpb, (unsigned)red.max_blocks);
-    k_bounce<S, R><<<(unsigned)sum.blocks, kTpb, 0, st>>>(p);
+    launch(k_bounce<S, R>, (unsigned)sum.blocks, kTpb, to, p);
     return sum;
 }
 
@@ -915,9 +917,9 @@ void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStre
 
 #define EUP_INST(S, R)                                                                                 \
     template int launch_bc<S, R>(const Lat<S, R>&, const Geo&, const int*, const Phys<R>&, const HaloEdgesDevice&, \
-                                 cudaStream_t, bool, const ForceSum*);                                    \
+                                 const LaunchTo&, bool, const ForceSum*);                                    \
     template ForceSum launch_bounce<S, R>(const Lat<S, R>&, const Geo&, const LinksDevice&, const Reduce&, double*, \
-                                          int64_t, int64_t*, cudaStream_t);                            \
+                                          int64_t, int64_t*, const LaunchTo&);                         \
     template void launch_force<S, R>(const Lat<S, R>&, const Geo&, const LinksDevice&, const Reduce&, double*, \
                                      int64_t, int64_t*, cudaStream_t);                                 \
     template void launch_fill_xface<S, R>(const Lat<S, R>&, const Geo&, cudaStream_t);                 \

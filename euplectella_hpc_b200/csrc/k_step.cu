@@ -158,6 +158,7 @@ __device__ __forceinline__ int plane_of_block(const Geo& g) {
 template <typename S, typename R, bool DOWN>
 __global__ void __launch_bounds__(128) k_stream_collide_scalar(Lat<S, R> src, Lat<S, R> dst, Geo g, Phys<R> ph,
                                                                int i0, int ni) {
+    chain_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ni) return;
     node_step(src, dst, g, ph, i0 + t, (int)blockIdx.y + 1, plane_of_block<DOWN>(g));
@@ -387,6 +388,7 @@ __device__ __forceinline__ void pair_step(const Lat<S, float>& src, const Lat<S,
 template <typename S, int MINB, bool DOWN>
 __global__ void __launch_bounds__(128, MINB) k_stream_collide_pair(Lat<S, float> src, Lat<S, float> dst, Geo g,
                                                                    Phys<float> ph, PullBase<S> pb, int p0, int np) {
+    chain_begin();
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (t >= np) return;
     pair_step(src, dst, g, ph, pb, 2 * (p0 + t) + 1, (int)blockIdx.y + 1, plane_of_block<DOWN>(g));
@@ -420,7 +422,7 @@ bool sweep_down(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g) {
 
 template <typename S, typename R>
 bool launch_pair(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph, int occ, int part,
-                 cudaStream_t st) {
+                 const LaunchTo& to) {
     if constexpr (sizeof(R) != 4) {
         return false;
     } else {
@@ -447,7 +449,7 @@ bool launch_pair(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const
         if (part == kStreamFaces) {
             const int sides = g.l == 2 ? 1 : 2;
             const int64_t threads = (int64_t)sides * g.m * g.n;
-            k_stream_collide_pair_faces<S><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(src, dst, g, ph, pb,
+            k_stream_collide_pair_faces<S><<<(unsigned)((threads + 127) / 128), 128, 0, to.st>>>(src, dst, g, ph, pb,
                                                                                              sides);
             return true;
         }
@@ -459,18 +461,18 @@ bool launch_pair(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const
         // resident blocks of 128 threads per SM the register budget is sized for: by default
         // 6 (80 registers) for FP32 storage, 8 (64) for 16-bit storage, whose loads need fewer
         const int minb = occ > 0 ? occ + 3 : (sizeof(S) == 4 ? 6 : 8);
-        auto launch = [&](auto down) {
+        auto run = [&](auto down) {
             constexpr bool D = decltype(down)::value;
             switch (minb) {
-                case 4: k_stream_collide_pair<S, 4, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-                case 5: k_stream_collide_pair<S, 5, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-                case 6: k_stream_collide_pair<S, 6, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-                case 7: k_stream_collide_pair<S, 7, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
-                default: k_stream_collide_pair<S, 8, D><<<grid, bx, 0, st>>>(src, dst, g, ph, pb, p0, np); break;
+                case 4: launch(k_stream_collide_pair<S, 4, D>, grid, bx, to, src, dst, g, ph, pb, p0, np); break;
+                case 5: launch(k_stream_collide_pair<S, 5, D>, grid, bx, to, src, dst, g, ph, pb, p0, np); break;
+                case 6: launch(k_stream_collide_pair<S, 6, D>, grid, bx, to, src, dst, g, ph, pb, p0, np); break;
+                case 7: launch(k_stream_collide_pair<S, 7, D>, grid, bx, to, src, dst, g, ph, pb, p0, np); break;
+                default: launch(k_stream_collide_pair<S, 8, D>, grid, bx, to, src, dst, g, ph, pb, p0, np); break;
             }
         };
-        if (sweep_down(src, dst, g)) launch(std::true_type());
-        else launch(std::false_type());
+        if (sweep_down(src, dst, g)) run(std::true_type());
+        else run(std::false_type());
         return true;
     }
 }
@@ -620,7 +622,8 @@ bool launch_vec(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const 
 
 template <typename S, typename R>
 void launch_stream_collide(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph,
-                           int variant, cudaStream_t st, int part) {
+                           int variant, const LaunchTo& to, int part) {
+    const cudaStream_t st = to.st;
     // EUP_STEP_VARIANT bit 0: 16-byte vectors, bit 2: 8-byte vectors (when l allows), bit 3: one
     // node per thread, bits 4-6: occupancy target of the two-node kernel (n + 3 blocks per SM);
     // default: two nodes per thread (FP32 arithmetic, l even).  (Bit 12 concerns the halo: all
@@ -631,7 +634,7 @@ void launch_stream_collide(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo
         if ((variant & 1) && launch_vec<S, R, VW>(src, dst, g, ph, st)) return;
         if ((variant & 4) && launch_vec<S, R, (VW / 2 > 0 ? VW / 2 : 1)>(src, dst, g, ph, st)) return;
     }
-    if (!(variant & 8) && launch_pair<S, R>(src, dst, g, ph, (variant >> 4) & 7, part, st)) return;
+    if (!(variant & 8) && launch_pair<S, R>(src, dst, g, ph, (variant >> 4) & 7, part, to)) return;
     const int bx = 128;
     if (part == kStreamFaces) {
         const int sides = g.l == 1 ? 1 : 2;
@@ -643,18 +646,18 @@ void launch_stream_collide(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo
     const int ni = part == kStreamInterior ? g.l - 2 : g.l;
     if (ni <= 0) return;
     dim3 grid((ni + bx - 1) / bx, g.m, g.n);
-    if (sweep_down(src, dst, g)) k_stream_collide_scalar<S, R, true><<<grid, bx, 0, st>>>(src, dst, g, ph, i0, ni);
-    else k_stream_collide_scalar<S, R, false><<<grid, bx, 0, st>>>(src, dst, g, ph, i0, ni);
+    if (sweep_down(src, dst, g)) launch(k_stream_collide_scalar<S, R, true>, grid, bx, to, src, dst, g, ph, i0, ni);
+    else launch(k_stream_collide_scalar<S, R, false>, grid, bx, to, src, dst, g, ph, i0, ni);
 }
 
 template void launch_stream_collide<float, float>(const Lat<float, float>&, const Lat<float, float>&,
-                                                  const Geo&, const Phys<float>&, int, cudaStream_t, int);
+                                                  const Geo&, const Phys<float>&, int, const LaunchTo&, int);
 template void launch_stream_collide<double, double>(const Lat<double, double>&, const Lat<double, double>&,
-                                                    const Geo&, const Phys<double>&, int, cudaStream_t, int);
+                                                    const Geo&, const Phys<double>&, int, const LaunchTo&, int);
 template void launch_stream_collide<__half, float>(const Lat<__half, float>&, const Lat<__half, float>&,
-                                                   const Geo&, const Phys<float>&, int, cudaStream_t, int);
+                                                   const Geo&, const Phys<float>&, int, const LaunchTo&, int);
 template void launch_stream_collide<__nv_bfloat16, float>(const Lat<__nv_bfloat16, float>&,
                                                           const Lat<__nv_bfloat16, float>&, const Geo&,
-                                                          const Phys<float>&, int, cudaStream_t, int);
+                                                          const Phys<float>&, int, const LaunchTo&, int);
 
 }  // namespace eup
