@@ -1650,9 +1650,10 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
                     const Lat<S, R> src = buf_lat(cur), dst = buf_lat(next);
                     const uint64_t key = ((uint64_t)1 << 60) | ((uint64_t)cur << 24) | (uint64_t)next;
                     const cudaError_t e_run = step(key, [&] {
-                        launch_bc<S, R>(src, g, bc, ph, h->edges, st, bc_separate(h));
+                        const LaunchTo to(st, graphs);
+                        launch_bc<S, R>(src, g, bc, ph, h->edges, to, bc_separate(h));
                         launch_pbb_step<S, R>(src, dst, g, ph, ns, h->ns_list, h->ns_count, red, nullptr, 0, nullptr,
-                                              st);
+                                              to);
                     });
                     CK(h, e_run);
                     cur = next;

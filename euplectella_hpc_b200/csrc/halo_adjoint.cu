@@ -73,7 +73,7 @@ __global__ void k_emit(Geo g, Faces p, int64_t items, uint64_t* key_c, uint64_t*
             g.shell_node(s - (int64_t)q * g.G, &i, &j, &k);
             there = g.interior(i + cx_of(q), j + cy_of(q), k + cz_of(q));
         }
-        if (there && kind <= kEdgeCopyMinus) kc = (uint64_t)q_src * (uint64_t)g.N + (uint64_t)src;
+        if (there && kind <= kEdgeCopyMinus) kc = (uint64_t)q_src << 32 | (uint64_t)src;
         // the population produced: the free-slip rim moves it to another population's slot
         if (there && kind == kEdgeOutflow) ko = (uint64_t)src << 5 | (uint64_t)(9 + q_src);
         key_c[t] = kc;
@@ -199,7 +199,7 @@ cudaError_t build_halo_adjoint(const Geo& g, const int bc[6], const HaloEdgesDev
     int h_runs[2] = {0, 0};
     int* run_len = reinterpret_cast<int*>(key1);
     if (e == cudaSuccess && nc > 0) {
-        e = sorted(key_c, (uint64_t)Q * (uint64_t)g.N);
+        e = sorted(key_c, (uint64_t)Q << 32);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(const_cast<int64_t*>(out->copy_slot), slot2, sizeof(int64_t) * nc,
                                 cudaMemcpyDeviceToDevice, st);

@@ -310,7 +310,7 @@ int64_t compact_flags(const uint8_t* flags, int64_t n, int32_t* out, void* scrat
 
 // ---- partial bounce-back and its adjoint (k_adjoint.cu) -------------------------
 // Where the adjoint of each halo value goes, on the device.  copy_*: halo slots holding a copy of
-// an interior population, grouped by source key q*N + lin (CSR: copy_start), ascending within a
+// an interior population, grouped by source key q << 32 | lin (CSR: copy_start), ascending within a
 // group.  out_*: halo slots holding an outflow equilibrium, grouped by the x = l node
 // (j-1) + (k-1)*m they are computed from, with the population produced, by population and slot.
 struct HaloAdjointDevice {

@@ -78,10 +78,16 @@ __device__ __forceinline__ R pull_pre(const Lat<R, R>& L, const Geo& g, int q, i
 // momentum the solid takes, F = sum 2 n_s j(x) over the list, j the momentum of the pulled
 // populations, in FP64 into series[(itime + 1) % cap], advancing the device step counter
 // (one block at least, so an empty list records a zero force).
+//
+// A voxel reads 38 values in 38 places: the loads in flight count, and behind them three
+// dependent latencies and the sum.  The register budget keeps five (16-bit storage), four or
+// (FP64) three blocks of 128 on an SM; the FP64 momentum takes the signed terms alone.  A
+// partial-bounce-back step at 192x96x96 (270 000 voxels listed), blocks of 256 with the products by
+// zero components / this: FP16 93.9 / 87.4 us, FP64 142.9 / 134.7, FP32 no change (82).
 template <typename S, typename R>
-__global__ void __launch_bounds__(256) k_pbb_list(Lat<S, R> src, Lat<S, R> dst, Geo g, const R* ns,
-                                                  const int32_t* list, int64_t nlist, Reduce red, double* series,
-                                                  int64_t cap, int64_t* d_itime) {
+__global__ void __launch_bounds__(128, sizeof(S) == 2 ? 5 : (sizeof(S) == 4 ? 4 : 3)) k_pbb_list(
+    Lat<S, R> src, Lat<S, R> dst, Geo g, const R* ns, const int32_t* list, int64_t nlist, Reduce red, double* series,
+    int64_t cap, int64_t* d_itime) {
     chain_begin();
     using P = PState<S, R>;
     double f[3] = {0.0, 0.0, 0.0};
@@ -105,10 +111,11 @@ __global__ void __launch_bounds__(256) k_pbb_list(Lat<S, R> src, Lat<S, R> dst, 
         if (series) {
             double jx = 0.0, jy = 0.0, jz = 0.0;
 #pragma unroll
-            for (int q = 0; q < 19; ++q) {
-                jx += (q == 18 ? 0 : cx_of(q)) * (double)pre[q];
-                jy += (q == 18 ? 0 : cy_of(q)) * (double)pre[q];
-                jz += (q == 18 ? 0 : cz_of(q)) * (double)pre[q];
+            for (int q = 0; q < 18; ++q) {
+                const double v = (double)pre[q];
+                if (cx_of(q) != 0) jx = cx_of(q) > 0 ? jx + v : jx - v;
+                if (cy_of(q) != 0) jy = cy_of(q) > 0 ? jy + v : jy - v;
+                if (cz_of(q) != 0) jz = cz_of(q) > 0 ? jz + v : jz - v;
             }
             // sum_q c_q w_q = 0: the momentum of the deviations is the momentum
             const double js = P::dev ? 1.0 / (double)src.scale : 1.0;
@@ -296,33 +303,46 @@ __global__ void __launch_bounds__(128) k_pbb_adjoint_faces(Lat<S, R> f, Geo g, P
 }
 
 // Halo values copied from interior populations: add their adjoints back, one
-// thread per source, sources' halo slots summed in a fixed order.
+// thread per source, sources' halo slots summed in a fixed order.  A chain of four dependent
+// loads bounds it; the source comes as population and node, not as a product to divide.
 template <typename R>
-__global__ void k_adj_copy(Geo g, const int64_t* key, const int32_t* start, const int64_t* slot, int64_t nkey,
-                           const R* gmu, Lat<R, R> lam_out) {
+__global__ void __launch_bounds__(128) k_adj_copy(const int64_t* key, const int32_t* start, const int64_t* slot,
+                                                  int64_t nkey, const R* gmu,
+                                                  const __grid_constant__ Lat<R, R> lam_out) {
+    chain_begin();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nkey) return;
+    const int64_t k = key[t];
+    const int32_t e0 = start[t], e1 = start[t + 1];
+    R* at = lam_out.pop[k >> 32] + (uint32_t)k;
+    const R old = *at;
     R acc = R(0);
-    for (int32_t e = start[t]; e < start[t + 1]; ++e) acc += gmu[slot[e]];
-    const int q = (int)(key[t] / g.N);
-    const int64_t lin = key[t] % g.N;
-    lam_out.pop[q][lin] += acc;
+    for (int32_t e = e0; e < e1; ++e) acc += gmu[slot[e]];
+    *at = old + acc;
 }
 
 // Outflow halo values (equilibria of the momentum of x = l,
 // CODE/SRC/bcond.bc.F90:138-165): propagate their adjoints to the 18 moving
-// populations of the node they were computed from.
+// populations of the node they were computed from.  The state's column comes from its x-face
+// copy (the same values, coalesced).
 template <typename S, typename R>
-__global__ void k_adj_outflow(Geo g, const int32_t* jk, const int32_t* start, const int64_t* slot, const int8_t* qo,
-                              int64_t nsrc, const R* gmu, Lat<S, R> f, Lat<R, R> lam_out) {
+__global__ void __launch_bounds__(64) k_adj_outflow(Geo g, const int32_t* jk, const int32_t* start, const int64_t* slot,
+                                                    const int8_t* qo, int64_t nsrc, const R* gmu, Lat<S, R> f,
+                                                    Lat<R, R> lam_out) {
+    chain_begin();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nsrc) return;
-    const int j = jk[t] % g.m + 1, k = jk[t] / g.m + 1;
-    const int64_t lin = g.lin(g.l, j, k);
-    R J[3] = {R(0), R(0), R(0)};
-    R a[18];
+    const int64_t row = jk[t];
+    const int64_t lin = (g.l - 1) + g.l * row;
+    R a[18], old[18];
+    const R* col = f.xface + (g.xs + g.xr + row);
 #pragma unroll
-    for (int q = 0; q < 18; ++q) a[q] = PState<S, R>::f_of(f, q, lin);
+    for (int q = 0; q < 18; ++q) a[q] = col[xface_slot(q) * g.mn];
+    // all 18 values of the node first, then the updated ones (a load after a store through
+    // another population's pointer would wait for it)
+#pragma unroll
+    for (int p = 0; p < 18; ++p) old[p] = lam_out.pop[p][lin];
+    R J[3];
     J[0] = a[0] + a[1] + a[2] + a[3] + a[4] - a[9] - a[10] - a[11] - a[12] - a[13];
     J[1] = a[2] + a[6] + a[7] + a[8] + a[11] - a[0] - a[9] - a[15] - a[16] - a[17];
     J[2] = a[3] + a[5] + a[6] + a[12] + a[17] - a[1] - a[8] - a[10] - a[14] - a[15];
@@ -335,11 +355,6 @@ __global__ void k_adj_outflow(Geo g, const int32_t* jk, const int32_t* start, co
         const R w = weight<R>(q);
         for (int a3 = 0; a3 < 3; ++a3) psi[a3] += mu * w * (R(3) * c[a3] + R(1.5) * (R(6) * cJ * c[a3] - R(2) * J[a3]));
     }
-    // all 18 values of the node first, then the updated ones (a load after a store through
-    // another population's pointer would wait for it)
-    R old[18];
-#pragma unroll
-    for (int p = 0; p < 18; ++p) old[p] = lam_out.pop[p][lin];
 #pragma unroll
     for (int p = 0; p < 18; ++p)
         lam_out.pop[p][lin] = old[p] + (R(cx_of(p)) * psi[0] + R(cy_of(p)) * psi[1] + R(cz_of(p)) * psi[2]);
@@ -359,7 +374,7 @@ void launch_pbb_step(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, c
                      const int32_t* ns_list, int64_t ns_count, const Reduce& red, double* series, int64_t cap,
                      int64_t* d_itime, const LaunchTo& to) {
     launch_stream_collide<S, R>(src, dst, g, ph, 0, to);
-    launch(k_pbb_list<S, R>, capped_grid(ns_count, 256), 256, to, src, dst, g, ns, ns_list, ns_count, red, series, cap,
+    launch(k_pbb_list<S, R>, capped_grid(ns_count, 128), 128, to, src, dst, g, ns, ns_list, ns_count, red, series, cap,
            d_itime);
 }
 
@@ -384,12 +399,12 @@ void launch_pbb_adjoint(const Lat<S, R>& f, const Geo& g, const Phys<R>& ph, con
     }
     if (!(parts & kAdjTransposes)) return;
     if (t.ncopy > 0)
-        // small blocks: a few thousand threads still spread over every SM
-        k_adj_copy<R><<<(unsigned)((t.ncopy + 63) / 64), 64, 0, st>>>(g, t.copy_key, t.copy_start, t.copy_slot,
-                                                                       t.ncopy, gmu, lam_out);
+        launch(k_adj_copy<R>, (unsigned)((t.ncopy + 127) / 128), 128, LaunchTo(st), t.copy_key, t.copy_start, t.copy_slot,
+               t.ncopy, gmu, lam_out);
     if (t.nout > 0)
-        k_adj_outflow<S, R><<<(unsigned)((t.nout + 63) / 64), 64, 0, st>>>(g, t.out_jk, t.out_start, t.out_slot,
-                                                                            t.out_q, t.nout, gmu, f, lam_out);
+        // small blocks: a few thousand threads still spread over every SM
+        launch(k_adj_outflow<S, R>, (unsigned)((t.nout + 63) / 64), 64, LaunchTo(st, t.ncopy > 0), g, t.out_jk,
+               t.out_start, t.out_slot, t.out_q, t.nout, gmu, f, lam_out);
 }
 
 #define EUP_PBB_INST(S, R)                                                                                       \

@@ -839,7 +839,8 @@ void launch_line(const Lat<S, R>& L, const Geo& g, int axis, int c1, int c2, dou
 }
 
 // Blocks of 128 threads: as many along x as a row fills, the rest over rows; enough shares for
-// a few waves of the 12 blocks an SM holds.
+// a few waves of the 12 blocks an SM holds, but eight rows a thread at least, so that the
+// partial sums stay below the size of the staging buffer they go to.
 static PlaneWalk plane_walk(const Geo& g, int axis, dim3* block, int* planes) {
     PlaneWalk w;
     const int tx = g.l > 64 ? 128 : (g.l > 32 ? 64 : 32);
@@ -850,7 +851,7 @@ static PlaneWalk plane_walk(const Geo& g, int axis, dim3* block, int* planes) {
     w.xblocks = (g.l + tx - 1) / tx;
     w.plane = axis == 1 ? 1 : g.m;
     w.row = axis == 1 ? g.m : 1;
-    const int64_t most = (w.rows + (int)block->y - 1) / (int)block->y;
+    const int64_t most = w.rows / (8 * (int)block->y);
     const int64_t want = 148 * 12 * (axis == 0 ? 1 : 3) / ((int64_t)*planes * w.xblocks);
     w.shares = (int)std::max<int64_t>(1, std::min(most, want));
     return w;
