@@ -7,7 +7,6 @@
 #include <cstring>
 #include <string>
 #include <type_traits>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/eup.h"
@@ -1407,44 +1406,6 @@ int revolve_repetition(int64_t n, int64_t c) {
 
 enum : int { kActAdvance = 0, kActSnapshot = 1, kActRestore = 2, kActAdjoint = 3 };
 
-// CUDA graphs of the launch sequences an adjoint run repeats (a forward step between two given
-// buffers, an adjoint step from a given buffer), captured the first time a key is met and
-// launched from then on: a reverse sweep uses a few hundred distinct sequences thousands of
-// times.  With use == false the sequence is launched directly.
-struct GraphCache {
-    std::unordered_map<uint64_t, cudaGraphExec_t> exec;
-    ~GraphCache() {
-        for (auto& kv : exec) cudaGraphExecDestroy(kv.second);
-    }
-    // Captures (on st, which may hold pending work) and instantiates the sequence of key.
-    template <typename F>
-    cudaError_t prepare(uint64_t key, cudaStream_t st, F&& enqueue) {
-        if (exec.count(key)) return cudaSuccess;
-        cudaGraph_t graph = nullptr;
-        cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return e;
-        enqueue();
-        e = cudaStreamEndCapture(st, &graph);
-        if (e != cudaSuccess) return e;
-        cudaGraphExec_t ge = nullptr;
-        // kernels keep the priority of the stream they were captured from
-        e = cudaGraphInstantiate(&ge, graph, cudaGraphInstantiateFlagUseNodePriority);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) return e;
-        exec.emplace(key, ge);
-        return cudaSuccess;
-    }
-    template <typename F>
-    cudaError_t run(uint64_t key, cudaStream_t st, bool use, F&& enqueue) {
-        if (!use) {
-            enqueue();
-            return cudaGetLastError();
-        }
-        const cudaError_t e = prepare(key, st, enqueue);
-        if (e != cudaSuccess) return e;
-        return cudaGraphLaunch(exec.find(key)->second, st);
-    }
-};
 struct RevAct {
     int kind, arg;  // advance: steps; snapshot/restore: slot; adjoint: the step t reversed (from state t-1)
 };
@@ -1599,15 +1560,13 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
     // ---- forward sweep (the handle's own state, force series recorded) ----
     const int64_t t0 = h->itime;
     const int w0 = slots, w1 = slots + 1;  // the working buffers
-    // every step as a CUDA graph (EUP_STEP_VARIANT bit 1: plain launches): the forward sweep
-    // uses the handle's own step graphs, the reverse sweep the cache below
+    // the forward sweep uses the handle's own step graphs (EUP_STEP_VARIANT bit 1: plain launches)
     const bool graphs = !(h->variant & 2);
     int per_step = 0;
     if (graphs) {
         const cudaError_t e_cap = capture_graphs<S, R>(h, &per_step);
         CK(h, e_cap);
     }
-    GraphCache cache;
     CK(h, cudaEventRecord(ev[0], st));
     for (int s = 0; s < T; ++s) {
         if (store_at[(size_t)s] >= 0) CK(h, keep(store_at[(size_t)s]));
@@ -1628,17 +1587,16 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
     CK(h, cudaGetLastError());
 
     // ---- reverse sweep: the rest of the schedule ----
-    // Walked twice: first without launching, capturing and instantiating every distinct step
-    // graph while the device still runs the forward sweep, then enqueueing the steps behind it.
+    // Plain launches, chained where a step follows a step: a forward step is three launches and
+    // an adjoint step five, which the host enqueues faster than the smallest lattice runs them,
+    // where capturing and instantiating a graph for every pair of buffers cost more than the
+    // replays gained: eup_adjoint_run at 48x24x12 FP64, 150 steps, 20.0 / 13.5 ms with graphs /
+    // without; at 192x96x96 FP32, 400 steps, 157 / 143 ms.
     // The sweep needs nothing from the host's reading of the objective, which comes after.
     int64_t recomputed = 0;
-    auto reverse = [&](bool dry) -> int {
+    auto reverse = [&]() -> int {
         int cur = w0;           // buffer holding the working state (state T-1 now)
         int cur_lam = 0;        // lam[cur_lam] = adjoint of the state after the step being reversed
-        auto step = [&](uint64_t key, auto&& enqueue) -> cudaError_t {
-            if (!dry) return cache.run(key, st, graphs, enqueue);
-            return graphs ? cache.prepare(key, st, enqueue) : cudaSuccess;
-        };
         for (size_t a = first_adj; a < acts.size(); ++a) {
             const RevAct act = acts[a];
             if (act.kind == kActAdvance) {
@@ -1648,26 +1606,20 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
                 for (int s = 0; s < act.arg; ++s) {
                     const int next = (s + 1 == act.arg && target >= 0) ? target : (cur == w0 ? w1 : w0);
                     const Lat<S, R> src = buf_lat(cur), dst = buf_lat(next);
-                    const uint64_t key = ((uint64_t)1 << 60) | ((uint64_t)cur << 24) | (uint64_t)next;
-                    const cudaError_t e_run = step(key, [&] {
-                        const LaunchTo to(st, graphs);
-                        launch_bc<S, R>(src, g, bc, ph, h->edges, to, bc_separate(h));
-                        launch_pbb_step<S, R>(src, dst, g, ph, ns, h->ns_list, h->ns_count, red, nullptr, 0, nullptr,
-                                              to);
-                    });
-                    CK(h, e_run);
+                    const LaunchTo to(st, !serial);
+                    launch_bc<S, R>(src, g, bc, ph, h->edges, to, bc_separate(h));
+                    launch_pbb_step<S, R>(src, dst, g, ph, ns, h->ns_list, h->ns_count, red, nullptr, 0, nullptr, to);
+                    CK(h, cudaGetLastError());
                     cur = next;
-                    if (!dry) ++recomputed;
+                    ++recomputed;
                 }
                 if (target >= 0) ++a;  // the store is done
             } else if (act.kind == kActSnapshot) {
                 if (cur != act.arg) {  // not reached in these schedules: a store always follows a forward step
-                    if (!dry) {
-                        CK(h, cudaMemcpyAsync(bufs.p + state * act.arg, bufs.p + state * cur, sizeof(S) * state,
-                                              cudaMemcpyDeviceToDevice, st));
-                        CK(h, cudaMemcpyAsync(xfaces.p + xfs * act.arg, xfaces.p + xfs * cur, sizeof(R) * xfs,
-                                              cudaMemcpyDeviceToDevice, st));
-                    }
+                    CK(h, cudaMemcpyAsync(bufs.p + state * act.arg, bufs.p + state * cur, sizeof(S) * state,
+                                          cudaMemcpyDeviceToDevice, st));
+                    CK(h, cudaMemcpyAsync(xfaces.p + xfs * act.arg, xfaces.p + xfs * cur, sizeof(R) * xfs,
+                                          cudaMemcpyDeviceToDevice, st));
                     cur = act.arg;
                 }
             } else if (act.kind == kActRestore) {
@@ -1679,35 +1631,30 @@ int adjoint_run(eup_handle* h, const eup_adjoint_config* ac, double* objective, 
                                 lout = lat_at<R, R>(h, lam.p + state * (cur_lam ^ 1));
                 const bool in_window = t > T - A;
                 const R gam = in_window ? (R)gamma : R(0);
-                const uint64_t key = ((uint64_t)2 << 60) | ((uint64_t)cur << 24) | ((uint64_t)cur_lam << 1) |
-                                     (uint64_t)in_window;
-                const cudaError_t e_run = step(key, [&] {
-                    if (serial) {
-                        launch_bc<S, R>(f, g, bc, ph, h->edges, st, bc_separate(h));  // the halo of step t, from state t-1
-                        launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, st, kAdjAll);
-                        return;
-                    }
+                if (serial) {
+                    launch_bc<S, R>(f, g, bc, ph, h->edges, st, bc_separate(h));  // the halo of step t, from state t-1
+                    launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, st, kAdjAll);
+                } else {
                     // the interior nodes read no halo value and write other slots than the
                     // boundary-plane nodes: the halo of step t (from state t-1) and the boundary-plane
                     // nodes run on the side stream beside them; the halo transposes after both
-                    cudaEventRecord(side.fork, st);
-                    cudaStreamWaitEvent(side.s, side.fork, 0);
+                    CK(h, cudaEventRecord(side.fork, st));
+                    CK(h, cudaStreamWaitEvent(side.s, side.fork, 0));
                     launch_bc<S, R>(f, g, bc, ph, h->edges, side.s, bc_separate(h));
                     launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, side.s, kAdjFaces);
-                    cudaEventRecord(side.join, side.s);
+                    CK(h, cudaEventRecord(side.join, side.s));
                     launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, st, kAdjInterior);
-                    cudaStreamWaitEvent(st, side.join, 0);
+                    CK(h, cudaStreamWaitEvent(st, side.join, 0));
                     launch_pbb_adjoint<S, R>(f, g, ph, ns, lin_, lout, gmu.p, grad.p, gam, td, st, kAdjTransposes);
-                });
-                CK(h, e_run);
+                }
+                CK(h, cudaGetLastError());
                 cur_lam ^= 1;
             }
         }
         return EUP_OK;
     };
-    int rc = reverse(true);
-    if (rc == EUP_OK) rc = reverse(false);
-    if (rc != EUP_OK) {
+    if (const int rc = reverse()) {
+        if (side.s) cudaStreamSynchronize(side.s);
         cudaStreamSynchronize(st);
         return rc;
     }
