@@ -280,12 +280,14 @@ template <typename S, typename R>
 void launch_probes(const Lat<S, R>& L, const Geo& g, int npts, const int32_t* ijk, double* out,
                    cudaStream_t st);
 
-// Scatter one haloed host-layout array (T) into lattice population q + shell; a
-// value that is not finite sets bit q of *bad (device pointer).
+// Scatter nq haloed host-layout arrays (T), one behind the other, into lattice populations
+// q .. q+nq-1 and the shell; a value that is not finite sets its population's bit of *bad
+// (device pointer).
 template <typename S, typename R, typename T>
-void launch_scatter(const Lat<S, R>& L, const Geo& g, int q, const T* staging, unsigned int* bad, cudaStream_t st);
+void launch_scatter(const Lat<S, R>& L, const Geo& g, int q, int nq, const T* staging, unsigned int* bad,
+                    cudaStream_t st);
 template <typename S, typename R, typename T>
-void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStream_t st);
+void launch_gather(const Lat<S, R>& L, const Geo& g, int q, int nq, T* staging, cudaStream_t st);
 
 // Set-up kernels (k_setup.cu).
 void launch_build_mask(const int32_t* obs, const Geo& g, uint32_t* bits, int wpr, cudaStream_t st);

@@ -533,14 +533,18 @@ __global__ void k_probes(Lat<S, R> L, Geo g, int npts, const int32_t* ijk, doubl
 }
 
 // ---- host layout <-> device layout ------------------------------------------------------
-// Host values (T = float or double) into the lattice and the halo shell.  16-bit storage
+// Host values (T = float or double) of populations q0 + blockIdx.y into the lattice and the
+// halo shell, `stride` values apart.  16-bit storage
 // from double converts in double: f = w + D/scale is exact there, so a state downloaded as
 // double and uploaded again keeps every bit of D (through float, deviations below 2^-6
 // lose their low bits to the rounding of f).  A host value that is not finite sets bit q
 // of *bad (the caller rejects the state).
 template <typename S, typename R, typename T>
-__global__ void k_scatter(Lat<S, R> L, Geo g, int q, const T* src, int64_t total, unsigned int* bad) {
+__global__ void k_scatter(const __grid_constant__ Lat<S, R> L, Geo g, int q0, const T* from, int64_t stride,
+                          int64_t total, unsigned int* bad) {
     constexpr bool exact16 = DevStore<S>::value && sizeof(T) == 8;
+    const int q = q0 + (int)blockIdx.y;
+    const T* src = from + blockIdx.y * stride;
     const int64_t L2 = g.l + 2, M2 = g.m + 2;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -561,8 +565,10 @@ __global__ void k_scatter(Lat<S, R> L, Geo g, int q, const T* src, int64_t total
 
 // The lattice and halo shell as host values; 16-bit storage to double in double (exact).
 template <typename S, typename R, typename T>
-__global__ void k_gather(Lat<S, R> L, Geo g, int q, T* dst, int64_t total) {
+__global__ void k_gather(const __grid_constant__ Lat<S, R> L, Geo g, int q0, T* to, int64_t stride, int64_t total) {
     constexpr bool exact16 = DevStore<S>::value && sizeof(T) == 8;
+    const int q = q0 + (int)blockIdx.y;
+    T* dst = to + blockIdx.y * stride;
     const int64_t L2 = g.l + 2, M2 = g.m + 2;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -905,15 +911,16 @@ void launch_probes(const Lat<S, R>& L, const Geo& g, int npts, const int32_t* ij
 }
 
 template <typename S, typename R, typename T>
-void launch_scatter(const Lat<S, R>& L, const Geo& g, int q, const T* staging, unsigned int* bad, cudaStream_t st) {
+void launch_scatter(const Lat<S, R>& L, const Geo& g, int q, int nq, const T* staging, unsigned int* bad,
+                    cudaStream_t st) {
     const int64_t total = (int64_t)(g.l + 2) * (g.m + 2) * (g.n + 2);
-    k_scatter<S, R, T><<<grid_for(total, kTpb), kTpb, 0, st>>>(L, g, q, staging, total, bad);
+    k_scatter<S, R, T><<<dim3(grid_for(total, kTpb), nq), kTpb, 0, st>>>(L, g, q, staging, total, total, bad);
 }
 
 template <typename S, typename R, typename T>
-void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStream_t st) {
+void launch_gather(const Lat<S, R>& L, const Geo& g, int q, int nq, T* staging, cudaStream_t st) {
     const int64_t total = (int64_t)(g.l + 2) * (g.m + 2) * (g.n + 2);
-    k_gather<S, R, T><<<grid_for(total, kTpb), kTpb, 0, st>>>(L, g, q, staging, total);
+    k_gather<S, R, T><<<dim3(grid_for(total, kTpb), nq), kTpb, 0, st>>>(L, g, q, staging, total, total);
 }
 
 #define EUP_INST(S, R)                                                                                 \
@@ -938,12 +945,12 @@ void launch_gather(const Lat<S, R>& L, const Geo& g, int q, T* staging, cudaStre
                                        double*, cudaStream_t);                                         \
     template void launch_probes<S, R>(const Lat<S, R>&, const Geo&, int, const int32_t*, double*,      \
                                       cudaStream_t);                                                   \
-    template void launch_scatter<S, R, float>(const Lat<S, R>&, const Geo&, int, const float*,         \
+    template void launch_scatter<S, R, float>(const Lat<S, R>&, const Geo&, int, int, const float*,         \
                                               unsigned int*, cudaStream_t);                            \
-    template void launch_scatter<S, R, double>(const Lat<S, R>&, const Geo&, int, const double*,       \
+    template void launch_scatter<S, R, double>(const Lat<S, R>&, const Geo&, int, int, const double*,       \
                                                unsigned int*, cudaStream_t);                           \
-    template void launch_gather<S, R, float>(const Lat<S, R>&, const Geo&, int, float*, cudaStream_t); \
-    template void launch_gather<S, R, double>(const Lat<S, R>&, const Geo&, int, double*, cudaStream_t);
+    template void launch_gather<S, R, float>(const Lat<S, R>&, const Geo&, int, int, float*, cudaStream_t); \
+    template void launch_gather<S, R, double>(const Lat<S, R>&, const Geo&, int, int, double*, cudaStream_t);
 
 EUP_INST(float, float)
 EUP_INST(double, double)

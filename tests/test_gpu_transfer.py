@@ -55,3 +55,28 @@ def test_page_locked_transfers_equal_pageable(eup, require_gpu, prec):
         f_ref = s.forces()
     assert np.array_equal(out1, ref)
     assert np.array_equal(f, f_ref)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64", "fp16"])
+@pytest.mark.parametrize("size", [(3, 2, 1), (40, 24, 18), (150, 80, 60)], ids=["3x2x1", "40x24x18", "150x80x60"])
+@pytest.mark.parametrize("elem", [4, 8])
+def test_state_in_one_piece_and_in_nineteen(eup, require_gpu, prec, size, elem):
+    """Arrays one behind the other and arrays apart, small states (one launch and one copy or
+    nineteen) and one above the limit for that: what goes up comes down, halo included."""
+    l, m, n = size
+    code = {"fp32": eup.FP32, "fp64": eup.FP64, "fp16": eup.FP16_DEV}[prec]
+    dt = np.float32 if elem == 4 else np.float64
+    a = eup.init_equilibrium(l, m, n, 0.05, 1e-3, 21, dt)
+    with eup.Solver(eup.Config(l, m, n, svisc=0.05, u_inflow=0.05, precision=code)) as s:
+        s.upload(a)
+        whole = s.download(dt)
+        if prec == "fp64" or elem == 4 and prec == "fp32":
+            assert np.array_equal(whole, a)  # no rounding on the way
+        apart = [np.ascontiguousarray(a[q]) for q in range(19)]
+        s.upload_ptrs([x.ctypes.data for x in apart], elem)
+        back = [np.empty_like(a[0]) for _ in range(19)]
+        s.download_ptrs([x.ctypes.data for x in back], elem)
+        assert np.array_equal(np.stack(back), whole)
+        a[7, 0, 0, 0] = np.nan  # a halo value of population 8
+        with pytest.raises(eup.EupError, match="a8"):
+            s.upload(a)
