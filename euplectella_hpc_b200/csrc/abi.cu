@@ -45,6 +45,8 @@ struct eup_handle {
     double* series = nullptr;
     int64_t cap = 0;
     double* dscratch = nullptr;  // 64 doubles
+    double* force_host = nullptr; // page-locked: the force of the state of step force_itime
+    int64_t force_itime = -1;     // -1: force_host is not current
     unsigned int* d_bad = nullptr;  // upload check: bit q set when population q had a non-finite value
     void* staging = nullptr;
     size_t staging_bytes = 0;
@@ -152,7 +154,8 @@ Reduce make_reduce(const eup_handle* h) { return Reduce{h->partials, h->counter,
 template <typename S, typename R>
 void enqueue_drag_only(eup_handle* h) {
     launch_force<S, R>(make_lat<S, R>(h, h->cur), h->g, h->links, make_reduce(h), h->series, h->cap, h->d_itime,
-                       h->stream);
+                       h->force_host, h->stream);
+    h->force_itime = h->itime;
 }
 
 // Events bracketing the phases of each step when profiling: ev[4*s + p].
@@ -398,8 +401,12 @@ int finish_state(eup_handle* h, int64_t itime) {
     h->has_state = true;
     h->mid_step = false;
     h->interior_done = false;
-    if (h->pbb) CK(h, cudaMemsetAsync(h->series + 3 * (itime % h->cap), 0, 3 * sizeof(double), h->stream));
-    else DISPATCH(h, enqueue_drag_only, h);
+    if (h->pbb) {
+        CK(h, cudaMemsetAsync(h->series + 3 * (itime % h->cap), 0, 3 * sizeof(double), h->stream));
+        h->force_itime = -1;
+    } else {
+        DISPATCH(h, enqueue_drag_only, h);
+    }
     CK(h, cudaGetLastError());
     CK(h, cudaStreamSynchronize(h->stream));
     return EUP_OK;
@@ -582,6 +589,8 @@ int eup_create(const eup_config* cfg, eup_handle** out) {
     cudaMemsetAsync(h->series, 0, sizeof(double) * 3 * h->cap, h->stream);
     if ((e = cudaMalloc(&h->dscratch, sizeof(double) * 64)) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(scratch)"));
+    if ((e = cudaMallocHost(&h->force_host, sizeof(double) * 3)) != cudaSuccess)
+        return cleanup_fail(cuda_fail(h, e, "cudaMallocHost(force)"));
     if ((e = cudaMalloc(&h->d_bad, sizeof(unsigned int))) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(upload check)"));
     const size_t xface_bytes = (size_t)xface_elems(h->g) * h->rbytes;
@@ -617,6 +626,7 @@ int eup_destroy(eup_handle* h) {
                     h->staging2, const_cast<HaloEdge*>(h->edges.e)};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    if (h->force_host) cudaFreeHost(h->force_host);
     for (cudaEvent_t e : h->xev)
         if (e) cudaEventDestroy(e);
     if (h->xfer) cudaStreamDestroy(h->xfer);
@@ -1197,9 +1207,13 @@ int eup_get_force_series(eup_handle* h, int64_t first_step, int32_t count, doubl
                     "eup_get_force_series: steps " + std::to_string(first_step) + ".." +
                         std::to_string(first_step + count - 1) + " outside the recorded range " +
                         std::to_string(lo) + ".." + std::to_string(h->itime));
-    // copies behind the steps on their stream: one wait in all for a force read every step
     cudaError_t e = cudaSuccess;
-    for (int32_t c = 0; c < count && e == cudaSuccess;) {
+    // the force of the state reached is in host memory once the steps have run (every call that
+    // changes the state under halfway bounce-back ends with its force); others are copied behind
+    // the steps on their stream.  step(1) and its force at 64x32x8:
+    // 35 us with the copy, 24.5 without.
+    const bool latest = count == 1 && first_step == h->itime && first_step == h->force_itime;
+    for (int32_t c = latest ? count : 0; c < count && e == cudaSuccess;) {
         const int64_t t = first_step + c;
         const int64_t pos = t % h->cap;
         const int32_t run = (int32_t)std::min<int64_t>(count - c, h->cap - pos);
@@ -1210,6 +1224,7 @@ int eup_get_force_series(eup_handle* h, int64_t first_step, int32_t count, doubl
     const cudaError_t es = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return cuda_fail(h, e, "eup_get_force_series");
+    if (latest) std::memcpy(fxyz, h->force_host, sizeof(double) * 3);
     for (int64_t t = 0; t < 3 * (int64_t)count; ++t)
         if (!std::isfinite(fxyz[t]))
             return fail(h, EUP_ERR_DIVERGED,
@@ -1744,6 +1759,7 @@ int eup_set_solid_fraction(eup_handle* h, const double* ns) {
     if (rc) return rc;
     CK(h, cudaStreamSynchronize(h->stream));
     drop_graphs(h);
+    h->force_itime = -1;
     if (!ns) {
         if (h->ns) cudaFree(h->ns);
         if (h->ns_list) cudaFree(h->ns_list);

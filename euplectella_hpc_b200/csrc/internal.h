@@ -45,6 +45,10 @@ __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The same in two parts, for kernels that fetch what no kernel of a step writes (lists, indices)
+// while they wait: 0.6 us of a step.  A thread with nothing to do may return between the two.
+__device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Bit-packed solid mask: one bit per interior node, rows along x padded to
 // 32-bit words (wpr words per (j,k) row).
@@ -212,6 +216,7 @@ struct ForceSum {
     double* series;
     int64_t cap;
     int64_t* d_itime;
+    double* host;  // the sum also goes here (page-locked host memory), if not null
 };
 // Bounce-back on solid voxels touching fluid/halo (CODE/SRC/bcond.obs.F90) with partial sums of
 // the FP64 momentum-exchange force of the state it reads; the halo launch of the step adds
@@ -219,10 +224,11 @@ struct ForceSum {
 template <typename S, typename R>
 ForceSum launch_bounce(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
                        int64_t cap, int64_t* d_itime, const LaunchTo& to);
-// The force alone, of the state in L, in one launch; the step counter stays.
+// The force alone, of the state in L, in one launch, to the history and to `host` (page-locked);
+// the step counter stays.
 template <typename S, typename R>
 void launch_force(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
-                  int64_t cap, int64_t* d_itime, cudaStream_t st);
+                  int64_t cap, int64_t* d_itime, double* host, cudaStream_t st);
 
 // x-slab faces: the five populations crossing an x face, (m+2)(n+2) values each.
 template <typename S, typename R>

@@ -81,29 +81,37 @@ __device__ __forceinline__ void sum_partials(const ForceSum& a, bool advance) {
         f[2] += __ldcg(a.partials + 3 * b + 2);
     }
     const double s = block_sum3(f);  // every thread has read d_itime before thread 0 writes it
-    if (threadIdx.x < 3) a.series[3 * (t % a.cap) + threadIdx.x] = s;
+    if (threadIdx.x < 3) {
+        a.series[3 * (t % a.cap) + threadIdx.x] = s;
+        if (a.host) a.host[threadIdx.x] = s;
+    }
     if (advance && threadIdx.x == 0) *a.d_itime = t + 1;
 }
 
 template <typename S, typename R>
 __global__ void __launch_bounds__(kTpb) k_bounce(const __grid_constant__ BounceArgs<S, R> p) {
-    chain_begin();
+    chain_open();
     double f[3] = {0.0, 0.0, 0.0};
     const int64_t total = p.links.nfluid + p.links.nhalo;
-    for (int64_t t = (int64_t)blockIdx.x * kTpb + threadIdx.x; t < total; t += (int64_t)gridDim.x * kTpb) {
+    int64_t t = (int64_t)blockIdx.x * kTpb + threadIdx.x;
+    FluidLink k = {};  // of this pass, fetched during the one before, or during the wait
+    if (t < p.links.nfluid) k = p.links.fluid[t];
+    chain_wait();
+    for (; t < total; t += (int64_t)gridDim.x * kTpb) {
         int32_t lin;
         uint32_t e;
         S raw;
         R val, push;  // the value stored, and the one that pushes the solid
         bool counts = true;
         if (t < p.links.nfluid) {
-            const FluidLink k = p.links.fluid[t];
             lin = k.lin;
             e = k.q;
             raw = p.from[e & kLinkQ][lin];
             if constexpr (DevStore<S>::value) val = p.w[e & kLinkQ] + DevStore<S>::to_f(raw) * p.L.inv_scale;
             else val = raw;
             push = val;
+            const int64_t next = t + (int64_t)gridDim.x * kTpb;
+            if (next < p.links.nfluid) k = p.links.fluid[next];
         } else {
             const HaloLink k = p.links.halo[t - p.links.nfluid];
             lin = k.lin;
@@ -203,7 +211,7 @@ __device__ __forceinline__ void outflow_row(const Lat<S, R>& L, const Geo& g, in
 
 template <typename S, typename R>
 __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<S, R> p) {
-    chain_begin();
+    chain_open();
     int s = 0;
 #pragma unroll
     for (int i = 1; i < kHaloSegments; ++i) s += blockIdx.x >= p.first[i];
@@ -211,12 +219,14 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
     const unsigned t = (blockIdx.x - p.first[s]) * kTpb + threadIdx.x;
     if (t >= f.count) return;
     if (f.kind == kSegForce) {
+        chain_wait();
         sum_partials(p.sum, true);
         return;
     }
     R v[5];
     if (f.kind == kSegEdges) {
         const HaloEdge e = f.edges[t];
+        chain_wait();
         if (e.kind <= kEdgeCopyMinus) {
             v[0] = Store<S, R>::load(p.L.pop[e.q][e.src], e.q, p.L.inv_scale);
             if (e.kind == kEdgeCopyPlus) v[0] = v[0] + p.force;
@@ -234,6 +244,7 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
     }
     const unsigned b = t / f.na, a = t - b * f.na;
     const int64_t from = a + b * f.src_b, to = a + b * f.dst_b;
+    chain_wait();
     if (f.kind == kFaceOutflow) {
         outflow_row(p.L, p.g, from, v);
     } else if (f.kind == kFaceConst) {
@@ -798,7 +809,7 @@ BounceArgs<S, R> bounce_args(const Lat<S, R>& L, const Geo& g, const LinksDevice
 template <typename S, typename R>
 ForceSum launch_bounce(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
                        int64_t cap, int64_t* d_itime, const LaunchTo& to) {
-    ForceSum sum{red.partials, 0, series, cap, d_itime};
+    ForceSum sum{red.partials, 0, series, cap, d_itime, nullptr};
     if (links.nfluid + links.nhalo == 0) return sum;
     BounceArgs<S, R> p = bounce_args(L, g, links, red);
     p.bounce = 1;
@@ -809,11 +820,11 @@ ForceSum launch_bounce(const Lat<S, R>& L, const Geo& g, const LinksDevice& link
 
 template <typename S, typename R>
 void launch_force(const Lat<S, R>& L, const Geo& g, const LinksDevice& links, const Reduce& red, double* series,
-                  int64_t cap, int64_t* d_itime, cudaStream_t st) {
+                  int64_t cap, int64_t* d_itime, double* host, cudaStream_t st) {
     BounceArgs<S, R> p = bounce_args(L, g, links, red);
     p.finish = 1;
     p.sum = ForceSum{red.partials, (int)grid_for(links.nfluid + links.nhalo, kTpb, (unsigned)red.max_blocks), series,
-                     cap, d_itime};
+                     cap, d_itime, host};
     k_bounce<S, R><<<(unsigned)p.sum.blocks, kTpb, 0, st>>>(p);
 }
 
@@ -929,7 +940,7 @@ void launch_gather(const Lat<S, R>& L, const Geo& g, int q, int nq, T* staging, 
     template ForceSum launch_bounce<S, R>(const Lat<S, R>&, const Geo&, const LinksDevice&, const Reduce&, double*, \
                                           int64_t, int64_t*, const LaunchTo&);                         \
     template void launch_force<S, R>(const Lat<S, R>&, const Geo&, const LinksDevice&, const Reduce&, double*, \
-                                     int64_t, int64_t*, cudaStream_t);                                 \
+                                     int64_t, int64_t*, double*, cudaStream_t);                        \
     template void launch_fill_xface<S, R>(const Lat<S, R>&, const Geo&, cudaStream_t);                 \
     template void launch_pack_x<S, R>(const Lat<S, R>&, const Geo&, int, R*, cudaStream_t);              \
     template void launch_unpack_x<S, R>(const Lat<S, R>&, const Geo&, int, const R*, cudaStream_t);      \

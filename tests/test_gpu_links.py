@@ -38,3 +38,30 @@ def test_random_solids(eup, orc, require_gpu, prec, share, bc):
             got = s.download(dt)
             for q in range(19):
                 assert np.array_equal(got[q][keep], a[q][keep]), q + 1
+
+
+def test_force_reads_agree_across_models(eup, require_gpu):
+    """The force of the state reached (from host memory) and the same entry of the history, with
+    the partial-bounce-back model switched on and off in between."""
+    l, m, n = 24, 12, 8
+    obs = np.zeros((n, m, l), np.int32)
+    obs[2:5, 4:7, 8:11] = 1
+    a = eup.init_equilibrium(l, m, n, 0.05, 1e-3, 3, np.float32)
+    with eup.Solver(eup.Config(l, m, n, svisc=0.05, u_inflow=0.05)) as s:
+        s.set_obstacles(obs)
+        s.upload(a, 5)
+        for _ in range(3):
+            s.step(1)
+            assert np.array_equal(s.forces(), s.force_series(s.itime - 1, 2)[1])
+        s.set_obstacles(np.zeros_like(obs))
+        assert np.all(s.forces() == 0.0)
+        s.set_solid_fraction(np.full((n, m, l), 0.3))
+        s.upload(a, 8)
+        assert np.all(s.forces() == 0.0)  # a fresh state under this model has no recorded force
+        s.step(1)
+        f = s.forces()
+        assert f[0] != 0.0 and np.array_equal(f, s.force_series(8, 2)[1])
+        s.set_solid_fraction(None)
+        assert np.array_equal(s.forces(), f)
+        s.step(1)
+        assert np.all(s.forces() == 0.0) and s.itime == 10
