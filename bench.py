@@ -300,7 +300,7 @@ def run_eup(args):
     s_solver = torch.cuda.ExternalStream(solver.stream())
     clocks = ClockSampler(local)
     clocks.start()
-    # timed region: K time steps (each one CUDA-graph launch of the step's kernels)
+    # timed region: K time steps (CUDA-graph launches of the steps' kernels)
     launches0 = solver.launches
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     ev0.record(s_solver)
