@@ -338,15 +338,38 @@ struct HaloAdjointDevice {
 cudaError_t build_halo_adjoint(const Geo& g, const int bc[6], const HaloEdgesDevice& edges, HaloAdjointDevice* out,
                                std::string* err, cudaStream_t st);
 
+// Momentum the solid takes from a voxel of solid fraction s: 2 s j, j the momentum of the pulled
+// kernel values pre (of deviations the same, sum_q c_q w_q = 0) times js, in FP64, the signed
+// terms alone.
+template <typename R>
+__device__ __forceinline__ void pbb_momentum(const R (&pre)[19], R s, double js, double (&f)[3]) {
+    double jx = 0.0, jy = 0.0, jz = 0.0;
+#pragma unroll
+    for (int q = 0; q < 18; ++q) {
+        const double v = (double)pre[q];
+        if (cx_of(q) != 0) jx = cx_of(q) > 0 ? jx + v : jx - v;
+        if (cy_of(q) != 0) jy = cy_of(q) > 0 ? jy + v : jy - v;
+        if (cz_of(q) != 0) jz = cz_of(q) > 0 ? jz + v : jz - v;
+    }
+    f[0] += 2.0 * (double)s * (jx * js);
+    f[1] += 2.0 * (double)s * (jy * js);
+    f[2] += 2.0 * (double)s * (jz * js);
+}
+
+// The partial-bounce-back step as one kernel over every node.
+template <typename S, typename R>
+void launch_pbb_whole(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph, const R* ns,
+                      const Reduce& red, double* series, int64_t cap, int64_t* d_itime, const LaunchTo& to);
+
 // One partial-bounce-back step src -> dst (any storage; FP32 arithmetic for 16-bit storage):
-// the plain stream-collide, then the mixing f* = (1 - n_s) BGK(f) + n_s f_opp on the ns_count
-// voxels of ns_list (those with n_s > 0).  With `series` the FP64 force of the step goes to
+// with `whole` in one pass over every node, else the plain stream-collide, then the mixing
+// f* = (1 - n_s) BGK(f) + n_s f_opp on the ns_count voxels of ns_list (those with n_s > 0).  With `series` the FP64 force of the step goes to
 // series[(itime + 1) % cap] and the device step counter advances; series == nullptr skips it
 // (recomputation in the adjoint).
 template <typename S, typename R>
 void launch_pbb_step(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph, const R* ns,
-                     const int32_t* ns_list, int64_t ns_count, const Reduce& red, double* series, int64_t cap,
-                     int64_t* d_itime, const LaunchTo& to);
+                     const int32_t* ns_list, int64_t ns_count, bool whole, const Reduce& red, double* series,
+                     int64_t cap, int64_t* d_itime, const LaunchTo& to);
 // Adjoint of one partial-bounce-back step from state f (its halo shell holding the step's
 // halo values); the adjoint fields lam are in the arithmetic type.  The adjoint is pushed:
 // node x writes lam_out_q at the node x - c_q it pulled from, each slot once.  parts:

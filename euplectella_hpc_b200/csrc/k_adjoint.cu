@@ -70,7 +70,7 @@ __device__ __forceinline__ R pull_pre(const Lat<R, R>& L, const Geo& g, int q, i
     return PState<R, R>::pull_f(L, g, q, i, j, k, lin, face);
 }
 
-// The partial-bounce-back step is the plain stream-collide (every node's BGK value, the
+// The partial-bounce-back step in two passes is the plain stream-collide (every node's BGK value, the
 // same kernels and bits as the plain step) followed by this kernel over the list of
 // voxels with n_s > 0: it pulls their pre-collision populations again, mixes
 //   f*_q = (1 - n_s) BGK_q + n_s f_opp(q)
@@ -108,21 +108,7 @@ __global__ void __launch_bounds__(128, sizeof(S) == 2 ? 5 : (sizeof(S) == 4 ? 4 
 #pragma unroll
         for (int q = 0; q < 19; ++q) x[q] = P::kval(dst.pop[q][lin]);
         const R s = ns[lin], s1 = R(1) - s;
-        if (series) {
-            double jx = 0.0, jy = 0.0, jz = 0.0;
-#pragma unroll
-            for (int q = 0; q < 18; ++q) {
-                const double v = (double)pre[q];
-                if (cx_of(q) != 0) jx = cx_of(q) > 0 ? jx + v : jx - v;
-                if (cy_of(q) != 0) jy = cy_of(q) > 0 ? jy + v : jy - v;
-                if (cz_of(q) != 0) jz = cz_of(q) > 0 ? jz + v : jz - v;
-            }
-            // sum_q c_q w_q = 0: the momentum of the deviations is the momentum
-            const double js = P::dev ? 1.0 / (double)src.scale : 1.0;
-            f[0] += 2.0 * (double)s * (jx * js);
-            f[1] += 2.0 * (double)s * (jy * js);
-            f[2] += 2.0 * (double)s * (jz * js);
-        }
+        if (series) pbb_momentum(pre, s, P::dev ? 1.0 / (double)src.scale : 1.0, f);
 #pragma unroll
         for (int q = 0; q < 19; ++q) {
             const S v = P::kstore(s1 * x[q] + s * pre[opp_of(q)]);
@@ -371,8 +357,9 @@ unsigned capped_grid(int64_t work, int tpb) {
 
 template <typename S, typename R>
 void launch_pbb_step(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph, const R* ns,
-                     const int32_t* ns_list, int64_t ns_count, const Reduce& red, double* series, int64_t cap,
-                     int64_t* d_itime, const LaunchTo& to) {
+                     const int32_t* ns_list, int64_t ns_count, bool whole, const Reduce& red, double* series,
+                     int64_t cap, int64_t* d_itime, const LaunchTo& to) {
+    if (whole) return launch_pbb_whole<S, R>(src, dst, g, ph, ns, red, series, cap, d_itime, to);
     launch_stream_collide<S, R>(src, dst, g, ph, 0, to);
     launch(k_pbb_list<S, R>, capped_grid(ns_count, 128), 128, to, src, dst, g, ns, ns_list, ns_count, red, series, cap,
            d_itime);
@@ -409,7 +396,7 @@ void launch_pbb_adjoint(const Lat<S, R>& f, const Geo& g, const Phys<R>& ph, con
 
 #define EUP_PBB_INST(S, R)                                                                                       \
     template void launch_pbb_step<S, R>(const Lat<S, R>&, const Lat<S, R>&, const Geo&, const Phys<R>&, const R*, \
-                                        const int32_t*, int64_t, const Reduce&, double*, int64_t, int64_t*,        \
+                                        const int32_t*, int64_t, bool, const Reduce&, double*, int64_t, int64_t*,  \
                                         const LaunchTo&);                                                             \
     template void launch_pbb_adjoint<S, R>(const Lat<S, R>&, const Geo&, const Phys<R>&, const R*,                \
                                            const Lat<R, R>&, const Lat<R, R>&, R*, double*, R,                     \
