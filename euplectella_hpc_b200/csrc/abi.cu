@@ -13,6 +13,7 @@
 #include "../../include/eup.h"
 #include "geometry.h"
 #include "internal.h"
+#include "pbb_plan.h"
 
 using namespace eup;
 
@@ -71,7 +72,7 @@ struct eup_handle {
     void* ns = nullptr;           // solid fraction n_s per interior node, arithmetic type
     int32_t* ns_list = nullptr;   // interior linear indices with n_s > 0, ascending
     int64_t ns_count = 0;
-    bool ns_whole = false;  // a step takes every node in one pass (pbb_in_one_pass)
+    bool ns_whole = false;  // a step takes every node in one pass (pbb_plan.h)
     bool ns_again = false;  // likewise a step run again without its force
     int64_t launches = 0;  // kernels launched by the step calls (split steps and plane pack/unpack too)
     bool mid_step = false;  // eup_step_boundaries done, eup_step_stream pending
@@ -156,29 +157,8 @@ Mask make_mask(const eup_handle* h) { return Mask{h->bits, h->wpr}; }
 // EUP_STEP_VARIANT without bit 12: one launch per halo block instead of one for all.
 bool bc_separate(const eup_handle* h) { return !(h->variant & 4096); }
 
-// A partial-bounce-back step in one pass over every node, or as the plain stream-collide and a
-// second pass over the listed voxels (launch_pbb_step).  The second pass costs a launch and the
-// 32-byte sectors that its voxels lie in, the one pass a share of the plain step whatever the
-// field.  us per step, two passes / one:
-//   192x96x96, voxels anywhere, sectors of 8 nodes touched 8 %, 15 %, 28 %, 49 %, 73 %:
-//     FP32 74/83 86/84 103/85 114/86 119/87, FP64 120/131 138/132 168/132 193/133 211/133,
-//     FP16 79/98 82/100 82/102 97/104 116/105;  in a block: 15 % FP32 77/82 FP64 128/130
-//     FP16 78/96, 49 % 116/83 183/130 167/98
-//   384x192x192, anywhere 8 %, 15 %, 28 %, 49 %: FP32 518/518 619/522 728/527 827/530,
-//     FP16 372/548 430/559 478/575 564/588;  block 15 %, 49 %: FP32 469/512 715/512, FP16
-//     521/540 1181/554
-//   48x24x12, any field: FP32 15-18/9.5, FP64 16-19/11.5, FP16 26-33/11.5
-//   64x48x40 and 127x31x33, any field: FP32 17-20/13-16, FP64 20-22/18-20, FP16 26-31/18-21;
-//     96x48x48 (221k nodes): FP32 19/19, FP64 24/27, FP16 29/25
-// The steps that an adjoint runs again sum no force: at 192x96x96 with 18 % of the sectors touched
-// FP32 80/70, FP64 133/115, FP16 no difference.  So: one pass on small lattices, and for
-// fields that touch more than 3/16 (16-bit storage 3/8) of the sectors, without the force 1/8 (3/16).
-// EUP_STEP_VARIANT bit 13: always two passes, bit 14: always one.
-bool pbb_in_one_pass(const eup_handle* h, int64_t sectors, bool force) {
-    if (h->variant & (8192 | 16384)) return (h->variant & 16384) != 0;
-    if (h->g.N <= 131072) return true;
-    const int64_t sixteenths = (force ? 3 : 2) + (h->sbytes == 2 ? (force ? 3 : 1) : 0);
-    return 16 * sectors > sixteenths * ((h->g.N + 7) / 8);
+bool pbb_one_pass(const eup_handle* h, int64_t sectors, bool force) {
+    return pbb_in_one_pass(h->g.l, h->g.N, h->sbytes, h->variant, sectors, force, kReduceMaxBlocks);
 }
 
 Reduce make_reduce(const eup_handle* h) { return Reduce{h->partials, h->counter, kReduceMaxBlocks}; }
@@ -1827,8 +1807,8 @@ int eup_set_solid_fraction(eup_handle* h, const double* ns) {
             sectors += list.empty() || list.back() / 8 != t / 8;
             list.push_back((int32_t)t);
         }
-    h->ns_whole = pbb_in_one_pass(h, sectors, true);
-    h->ns_again = pbb_in_one_pass(h, sectors, false);
+    h->ns_whole = pbb_one_pass(h, sectors, true);
+    h->ns_again = pbb_one_pass(h, sectors, false);
     if (!h->ns) CK(h, cudaMalloc(&h->ns, h->rbytes * N));
     if (h->ns_list) cudaFree(h->ns_list);
     h->ns_list = nullptr;

@@ -10,6 +10,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "pbb_plan.h"
 
 namespace eup {
 
@@ -693,14 +694,8 @@ void launch_stream_collide(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo
 template <typename S, typename R>
 void launch_pbb_whole(const Lat<S, R>& src, const Lat<S, R>& dst, const Geo& g, const Phys<R>& ph, const R* ns,
                       const Reduce& red, double* series, int64_t cap, int64_t* d_itime, const LaunchTo& to) {
-    const int rows = g.m * g.n;
-    const int nbx = (g.l + 127) / 128;
-    const int bx = ((g.l + nbx - 1) / nbx + 31) / 32 * 32;
-    // as few rounds as the partial sums have room for, with equal numbers of rows
-    const int64_t most = series ? std::max(1, kReduceMaxBlocks / nbx) : rows;
-    const int rounds = (int)((rows + most - 1) / most);
-    const int slots = (rows + rounds - 1) / rounds;
-    launch(k_pbb_whole<S, R>, (unsigned)(nbx * slots), bx, to, src, dst, g, ph, ns, nbx, rounds,
+    const PbbSplit s = pbb_split(g.l, g.m * g.n, series ? red.max_blocks : 0);
+    launch(k_pbb_whole<S, R>, (unsigned)s.blocks(), s.threads, to, src, dst, g, ph, ns, s.nbx, s.each,
            (int)sweep_down(src, dst, g), red, series, cap, d_itime);
 }
 
