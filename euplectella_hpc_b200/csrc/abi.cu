@@ -476,6 +476,26 @@ bool one_behind_the_other(const void* const pops[19], size_t bytes) {
     return true;
 }
 
+// The 19 host arrays to or from `dev`, where they lie one behind the other: one copy where CUDA
+// takes the host range, else nineteen.  Adjoining arrays may be page-locked by themselves
+// (small page-locked allocations come one behind the other) or only in part, and a copy over
+// more than one such range is refused (cudaErrorInvalidValue) before it starts.
+cudaError_t copy_populations(char* dev, void* const host[19], size_t bytes, bool to_device, cudaStream_t st) {
+    const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    auto copy = [&](int q, size_t n) {
+        void* d = dev + q * bytes;
+        return to_device ? cudaMemcpyAsync(d, host[q], n, kind, st) : cudaMemcpyAsync(host[q], d, n, kind, st);
+    };
+    if (one_behind_the_other(host, bytes)) {
+        const cudaError_t e = copy(0, Q * bytes);
+        if (e != cudaErrorInvalidValue) return e;
+        cudaGetLastError();
+    }
+    cudaError_t e = cudaSuccess;
+    for (int q = 0; q < Q && e == cudaSuccess; ++q) e = copy(q, bytes);
+    return e;
+}
+
 int ensure_staging(eup_handle* h, size_t bytes) {
     if (h->staging_bytes >= bytes) return EUP_OK;
     if (h->staging) cudaFree(h->staging);
@@ -885,11 +905,7 @@ int eup_upload(eup_handle* h, const void* const pops[19], int32_t elem_bytes, in
     if (Q * bytes <= kBatchBytes) {
         if ((rc = ensure_staging(h, Q * bytes)) || (rc = begin_upload_check(h))) return rc;
         char* buf = static_cast<char*>(h->staging);
-        const int copies = one_behind_the_other(pops, bytes) ? 1 : Q;
-        cudaError_t e = cudaSuccess;
-        for (int c = 0; c < copies && e == cudaSuccess; ++c)
-            e = cudaMemcpyAsync(buf + c * bytes, pops[c], copies == 1 ? Q * bytes : bytes, cudaMemcpyHostToDevice,
-                                h->stream);
+        cudaError_t e = copy_populations(buf, const_cast<void* const*>(pops), bytes, true, h->stream);
         if (e == cudaSuccess) DISPATCH(h, upload_q, h, 0, Q, elem_bytes, buf);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) {
@@ -1022,11 +1038,8 @@ int eup_download(eup_handle* h, void* const pops[19], int32_t elem_bytes) {
         if ((rc = ensure_staging(h, Q * bytes))) return rc;
         char* buf = static_cast<char*>(h->staging);
         DISPATCH(h, download_q, h, 0, Q, elem_bytes, buf);
-        const int copies = one_behind_the_other(pops, bytes) ? 1 : Q;
         cudaError_t e = cudaGetLastError();
-        for (int c = 0; c < copies && e == cudaSuccess; ++c)
-            e = cudaMemcpyAsync(pops[c], buf + c * bytes, copies == 1 ? Q * bytes : bytes, cudaMemcpyDeviceToHost,
-                                h->stream);
+        if (e == cudaSuccess) e = copy_populations(buf, pops, bytes, false, h->stream);
         const cudaError_t es = cudaStreamSynchronize(h->stream);
         if (e == cudaSuccess) e = es;
         return e == cudaSuccess ? EUP_OK : cuda_fail(h, e, "eup_download");
