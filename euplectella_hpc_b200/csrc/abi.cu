@@ -12,6 +12,7 @@
 
 #include "../../include/eup.h"
 #include "geometry.h"
+#include "host_page.h"
 #include "internal.h"
 #include "pbb_plan.h"
 
@@ -20,7 +21,23 @@ using namespace eup;
 // Steps per graph of a long run (even: a run ends on the lattice it started from), and the run
 // length from which such a graph is made.
 constexpr int kChunkSteps = 16, kChunkFrom = 32;
-constexpr size_t kHostPage = 4096;
+// Reads of the latest force after which a handle gets the page for it (host_page.h): a read takes
+// 10 us less with it, the page 0.5 ms to make and release.
+constexpr int kPageReads = 32;
+
+struct CudaPage {
+    static bool register_page(void* p, size_t n) {
+        // made in the middle of a run: allowed while another stream of the program is captured
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const bool ok = cudaHostRegister(p, n, cudaHostRegisterMapped) == cudaSuccess;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return ok;
+    }
+    static bool device_pointer(void* p, void** d) { return cudaHostGetDevicePointer(d, p, 0) == cudaSuccess; }
+    static void unregister_page(void* p) { cudaHostUnregister(p); }
+    static void clear_error() { cudaGetLastError(); }
+};
 
 struct eup_handle {
     eup_config cfg{};
@@ -48,10 +65,9 @@ struct eup_handle {
     double* series = nullptr;
     int64_t cap = 0;
     double* dscratch = nullptr;  // 64 doubles
-    double* force_host = nullptr; // page-locked: the force of the state of step force_itime
-    double* force_dev = nullptr;  // where the device writes it
-    bool force_registered = false;
-    int64_t force_itime = -1;     // -1: force_host is not current
+    HostPage<CudaPage> force_page;  // the force of the state of step force_itime
+    int64_t force_itime = -1;       // -1: force_page is not current
+    int force_reads = 0;            // reads of the latest force without the page
     unsigned int* d_bad = nullptr;  // upload check: bit q set when population q had a non-finite value
     void* staging = nullptr;
     size_t staging_bytes = 0;
@@ -166,8 +182,8 @@ Reduce make_reduce(const eup_handle* h) { return Reduce{h->partials, h->counter,
 template <typename S, typename R>
 void enqueue_drag_only(eup_handle* h) {
     launch_force<S, R>(make_lat<S, R>(h, h->cur), h->g, h->links, make_reduce(h), h->series, h->cap, h->d_itime,
-                       h->force_dev, h->stream);
-    h->force_itime = h->itime;
+                       h->force_page.dev, h->stream);
+    h->force_itime = h->force_page.dev ? h->itime : -1;
 }
 
 // Events bracketing the phases of each step when profiling: ev[4*s + p].
@@ -621,15 +637,6 @@ int eup_create(const eup_config* cfg, eup_handle** out) {
     cudaMemsetAsync(h->series, 0, sizeof(double) * 3 * h->cap, h->stream);
     if ((e = cudaMalloc(&h->dscratch, sizeof(double) * 64)) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(scratch)"));
-    // a page of our own, registered: 0.3 ms, where the first cudaMallocHost of a process takes 1.5
-    // (and the last cudaFreeHost 0.5)
-    h->force_host = static_cast<double*>(std::aligned_alloc(kHostPage, kHostPage));
-    if (!h->force_host) return cleanup_fail(cuda_fail(h, cudaErrorMemoryAllocation, "force page"));
-    if ((e = cudaHostRegister(h->force_host, kHostPage, cudaHostRegisterMapped)) == cudaSuccess) {
-        h->force_registered = true;
-        e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&h->force_dev), h->force_host, 0);
-    }
-    if (e != cudaSuccess) return cleanup_fail(cuda_fail(h, e, "cudaHostRegister(force)"));
     if ((e = cudaMalloc(&h->d_bad, sizeof(unsigned int))) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(upload check)"));
     const size_t xface_bytes = (size_t)xface_elems(h->g) * h->rbytes;
@@ -665,8 +672,7 @@ int eup_destroy(eup_handle* h) {
                     h->staging2, const_cast<HaloEdge*>(h->edges.e)};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    if (h->force_registered) cudaHostUnregister(h->force_host);
-    std::free(h->force_host);
+    h->force_page.close();
     for (cudaEvent_t e : h->xev)
         if (e) cudaEventDestroy(e);
     if (h->xfer) cudaStreamDestroy(h->xfer);
@@ -1241,11 +1247,14 @@ int eup_get_force_series(eup_handle* h, int64_t first_step, int32_t count, doubl
                         std::to_string(first_step + count - 1) + " outside the recorded range " +
                         std::to_string(lo) + ".." + std::to_string(h->itime));
     cudaError_t e = cudaSuccess;
-    // the force of the state reached is in host memory once the steps have run (every call that
-    // changes the state under halfway bounce-back ends with its force); others are copied behind
-    // the steps on their stream.  step(1) and its force at 64x32x8:
+    // with the page, the force of the state reached is in host memory once the steps have run (every
+    // call that changes the state under halfway bounce-back ends with its force); others are
+    // copied behind the steps on their stream.  step(1) and its force at 64x32x8:
     // 35 us with the copy, 24.5 without.
-    const bool latest = count == 1 && first_step == h->itime && first_step == h->force_itime;
+    const bool last = count == 1 && first_step == h->itime;
+    const bool latest = last && first_step == h->force_itime;
+    if (last && !h->pbb && !h->force_page.dev && ++h->force_reads == kPageReads)
+        h->force_page.open();  // used from the next state on; without it every read is a copy
     for (int32_t c = latest ? count : 0; c < count && e == cudaSuccess;) {
         const int64_t t = first_step + c;
         const int64_t pos = t % h->cap;
@@ -1257,7 +1266,7 @@ int eup_get_force_series(eup_handle* h, int64_t first_step, int32_t count, doubl
     const cudaError_t es = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return cuda_fail(h, e, "eup_get_force_series");
-    if (latest) std::memcpy(fxyz, h->force_host, sizeof(double) * 3);
+    if (latest) std::memcpy(fxyz, h->force_page.host, sizeof(double) * 3);
     for (int64_t t = 0; t < 3 * (int64_t)count; ++t)
         if (!std::isfinite(fxyz[t]))
             return fail(h, EUP_ERR_DIVERGED,
