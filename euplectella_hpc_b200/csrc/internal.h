@@ -209,7 +209,8 @@ cudaError_t build_links(const Geo& g, const int bc[6], const int32_t* list, cons
                         LinksDevice* out, void* scratch, size_t scratch_bytes, cudaStream_t st);
 
 // Where a sum of the force goes: series[3 * (*d_itime % cap)]; `blocks` partial sums of the
-// bounce-back launch are added in their order, and the device step counter advances.
+// bounce-back launch (three each, for FP64 six) are added in their order, and
+// the device step counter advances.
 struct ForceSum {
     const double* partials;
     int blocks;

@@ -48,50 +48,95 @@ struct BounceArgs {
     ForceSum sum;
 };
 
-// Sum over the block in threads 0..2 (component = thread); kTpb threads, fixed order.
-__device__ __forceinline__ double block_sum3(double (&f)[3]) {
-    __shared__ double sh[kTpb / 32][3];
-#pragma unroll 1
-    for (int o = 16; o > 0; o >>= 1) {
-        f[0] += __shfl_down_sync(0xffffffffu, f[0], o);
-        f[1] += __shfl_down_sync(0xffffffffu, f[1], o);
-        f[2] += __shfl_down_sync(0xffffffffu, f[2], o);
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
-        sh[threadIdx.x >> 5][0] = f[0];
-        sh[threadIdx.x >> 5][1] = f[1];
-        sh[threadIdx.x >> 5][2] = f[2];
-    }
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x < 3)
+// A force is a small difference of large sums (the pressure on either side of a body), and the
+// links come population by population, so that a plain sum adds up one side before it meets the
+// other.  FP32 values do so exactly in FP64 (populations of 2^-6 and more: below 2^24).  FP64
+// values lost 2e-14 at 256x128x64, where voxel by voxel 1e-17 to 8e-15 are lost, so each is split at
+// 2^-24: the multiples add up exactly below 2^29, the rest, at most 2^-25 each, loses 2^-20 of what
+// the plain sum lost, and the two meet when the sum is complete.  (Values beyond 2^27 or below
+// 2^-25 add up as in a plain sum.)
+template <typename R>
+struct Force {
+    static constexpr int kSums = sizeof(R) == 8 ? 6 : 3;  // three sums, or three of multiples and three of the rest
+    static constexpr int kPad = sizeof(R) == 8 ? 8 : 4;
+    double v[kPad] = {};
+    __device__ __forceinline__ void add(const double (&c2)[3], double x) {
+        if constexpr (sizeof(R) == 8) {
+            const double grid = 402653184.0;  // 1.5 2^28: its last digit is worth 2^-24
+            const double hi = (x + grid) - grid, lo = x - hi;
 #pragma unroll
-        for (int w = 0; w < kTpb / 32; ++w) s += sh[w][threadIdx.x];
-    return s;
-}
-
-// One block: the partial forces in a fixed order into the force history.
-__device__ __forceinline__ void sum_partials(const ForceSum& a, bool advance) {
-    const int64_t t = *a.d_itime;
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < a.blocks; b += kTpb) {
-        f[0] += __ldcg(a.partials + 3 * b);
-        f[1] += __ldcg(a.partials + 3 * b + 1);
-        f[2] += __ldcg(a.partials + 3 * b + 2);
+            for (int c = 0; c < 3; ++c) {
+                v[c] += c2[c] * hi;
+                v[3 + c] += c2[c] * lo;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] += c2[c] * x;
+        }
     }
-    const double s = block_sum3(f);  // every thread has read d_itime before thread 0 writes it
-    if (threadIdx.x < 3) {
-        a.series[3 * (t % a.cap) + threadIdx.x] = s;
-        if (a.host) a.host[threadIdx.x] = s;
+    // The sums over the block, sum c in the lanes 32 / kPad * c of the first warp and the ones
+    // behind it; kTpb threads, fixed order.  Lanes that are 16, 8 and (eight sums) 4 apart trade
+    // halves of what they still hold: six or nine exchanges, where fifteen or thirty sum one by one.
+    __device__ __forceinline__ double block_sum() {
+        static_assert(kTpb / 32 == 8, "eight warps' sums");
+        constexpr int kLanes = 32 / kPad;  // to a sum
+        __shared__ double sh[kPad][kTpb / 32];
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int h = kPad / 2; h > 0; h >>= 1) {
+            const bool up = lane & (kLanes * h);
+#pragma unroll
+            for (int i = 0; i < h; ++i) {
+                const double give = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, kLanes * h);
+            }
+        }
+        double s = v[0];  // sum lane / kLanes of the lanes that many apart
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        __syncthreads();
+        if (lane % kLanes == 0) sh[lane / kLanes][threadIdx.x >> 5] = s;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            s = sh[lane / kLanes][lane % kLanes];
+            if constexpr (kLanes == 4) s += sh[lane / kLanes][4 + lane % kLanes];
+#pragma unroll
+            for (int o = kLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        }
+        return s;
+    }
+    // Which sum this thread has to store (-1: none).
+    static __device__ __forceinline__ int mine() {
+        constexpr int kLanes = 32 / kPad;
+        return threadIdx.x < kLanes * kSums && threadIdx.x % kLanes == 0 ? (int)threadIdx.x / kLanes : -1;
+    }
+};
+
+// One block: the partial sums of the force in a fixed order into the force history.
+template <typename R>
+__device__ __forceinline__ void sum_partials(const ForceSum& a, bool advance) {
+    constexpr int W = Force<R>::kSums;
+    const int64_t t = *a.d_itime;
+    Force<R> f;
+    for (int b = threadIdx.x; b < a.blocks; b += kTpb)
+#pragma unroll
+        for (int c = 0; c < W; ++c) f.v[c] += __ldcg(a.partials + W * b + c);
+    double s = f.block_sum();  // every thread has read d_itime before thread 0 writes it
+    if (threadIdx.x < 32) {
+        if constexpr (W == 6) s += __shfl_down_sync(0xffffffffu, s, 12);  // the rest of the same component
+        const int c = Force<R>::mine();
+        if (c >= 0 && c < 3) {
+            a.series[3 * (t % a.cap) + c] = s;
+            if (a.host) a.host[c] = s;
+        }
     }
     if (advance && threadIdx.x == 0) *a.d_itime = t + 1;
 }
 
 template <typename S, typename R>
-__global__ void __launch_bounds__(kTpb) k_bounce(const __grid_constant__ BounceArgs<S, R> p) {
+__global__ void __launch_bounds__(kTpb, sizeof(R) == 8 ? 6 : 8) k_bounce(const __grid_constant__ BounceArgs<S, R> p) {
     chain_open();
-    double f[3] = {0.0, 0.0, 0.0};
+    Force<R> f;
     const int64_t total = p.links.nfluid + p.links.nhalo;
     int64_t t = (int64_t)blockIdx.x * kTpb + threadIdx.x;
     FluidLink k = {};  // of this pass, fetched during the one before, or during the wait
@@ -132,15 +177,11 @@ __global__ void __launch_bounds__(kTpb) k_bounce(const __grid_constant__ BounceA
                 if (e & kLinkXLast) x[p.g.xs] = val;
             }
         }
-        if (counts) {
-            const double v = (double)push;
-            f[0] += p.c2[q][0] * v;
-            f[1] += p.c2[q][1] * v;
-            f[2] += p.c2[q][2] * v;
-        }
+        if (counts) f.add(p.c2[q], (double)push);
     }
-    const double s = block_sum3(f);
-    if (threadIdx.x < 3) p.partials[3 * (int64_t)blockIdx.x + threadIdx.x] = s;
+    const double s = f.block_sum();
+    const int c = Force<R>::mine();
+    if (c >= 0) p.partials[Force<R>::kSums * (int64_t)blockIdx.x + c] = s;
     if (!p.finish) return;
     __shared__ bool last;
     __threadfence();
@@ -149,7 +190,7 @@ __global__ void __launch_bounds__(kTpb) k_bounce(const __grid_constant__ BounceA
     __syncthreads();
     if (!last) return;
     __threadfence();
-    sum_partials(p.sum, false);
+    sum_partials<R>(p.sum, false);
     if (threadIdx.x == 0) *p.counter = 0u;
 }
 
@@ -220,7 +261,7 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
     if (t >= f.count) return;
     if (f.kind == kSegForce) {
         chain_wait();
-        sum_partials(p.sum, true);
+        sum_partials<R>(p.sum, true);
         return;
     }
     R v[5];
