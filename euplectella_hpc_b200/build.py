@@ -25,7 +25,7 @@ LIB = os.path.join(LIB_DIR, "libeup.so")
 DRIVER = os.path.join(LIB_DIR, "eup_bgk3d")
 
 SOURCES = ["abi.cu", "k_bc.cu", "halo_plan.cu", "halo_adjoint.cu", "k_step.cu", "k_setup.cu", "k_adjoint.cu", "host.cpp", "noalloc.cu"]
-HEADERS = ["lbm_common.cuh", "internal.h", "geometry.h", "halo.h", "host_page.h", "init_eq.h", "pbb_plan.h"]
+HEADERS = ["lbm_common.cuh", "internal.h", "geometry.h", "halo.h", "host_page.h", "init_eq.h", "pbb_plan.h", "row_walk.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC,-fopenmp,-Wall,-ffp-contract=off",
           "-I", os.path.join(ROOT, "include")]

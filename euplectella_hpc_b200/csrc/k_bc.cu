@@ -8,6 +8,7 @@
 
 #include "halo.h"
 #include "internal.h"
+#include "row_walk.h"
 
 namespace eup {
 
@@ -316,9 +317,10 @@ __global__ void __launch_bounds__(kTpb) k_halo(const __grid_constant__ HaloPlan<
 
 // ---- FP64 monitor, CODE/SRC/diagno.F90:67-120 -------------------------------------------
 //
-// The diagnostics over all nodes walk the lattice by rows along x, a warp to a row: the loads of
-// every population are coalesced, the row index is all the mask needs (32 nodes share a word), and
-// no node pays for a division.  What bounds them is the read of the state, for 4- and 8-byte
+// The diagnostics over all nodes walk the lattice by rows along x, a warp to a row (row_walk.h: or to
+// a piece of a long one, or to several short ones): the loads of every population are
+// coalesced, the row index is all the mask needs (32 nodes share a word), and no node pays for
+// a division.  What bounds them is the read of the state, for 4- and 8-byte
 // storage; for 16-bit storage the conversions to FP64 and the FP64 adds.  Monitor, a thread per
 // node with three divisions / a warp per row: 298 / 232 us at 384x192x192 FP32, 2290 / 1560 at
 // 768x384x384, 5.3 / 3.3..3.8 ms at 1024x512x512 FP16.
@@ -343,21 +345,32 @@ __device__ __forceinline__ void node_sums(const Lat<S, R>& L, int64_t lin, doubl
     usq = xj * xj + yj * yj + zj * zj;
 }
 
-template <typename S, typename R>
-__global__ void __launch_bounds__(kTpb) k_monitor(Lat<S, R> L, int l, int64_t rows, Mask mk, Reduce red, double* out) {
-    double s[5] = {0, 0, 0, 0, 0};
-    const int lane = threadIdx.x & 31;
+// f(row, x) for every node, x from 0, by the warps of the grid.
+template <typename F>
+__device__ __forceinline__ void walk_rows(const RowWalk& w, F&& f) {
+    const int lane = threadIdx.x & 31, xl = lane & ((1 << w.lg) - 1);
     const int64_t step = (int64_t)gridDim.x * (kTpb / 32);
-    for (int64_t r = (int64_t)blockIdx.x * (kTpb / 32) + (threadIdx.x >> 5); r < rows; r += step)
-        for (int x = lane; x < l; x += 32) {
-            if (mk.bits != nullptr && (mk.bits[r * mk.wpr + (x >> 5)] >> lane) & 1u) {
-                s[0] += 1.0;
-                continue;
-            }
-            double rho, xj, yj, zj, usq;
-            node_sums(L, r * l + x, rho, xj, yj, zj, usq);
-            s[0] += rho; s[1] += xj; s[2] += yj; s[3] += zj; s[4] += usq;
+    for (int64_t u = (int64_t)blockIdx.x * (kTpb / 32) + (threadIdx.x >> 5); u < w.units; u += step) {
+        const int64_t group = w.pieces == 1 ? u : u / w.pieces;
+        const int first = (int)(u - group * w.pieces) * w.span, end = min(w.l - first, w.span);
+        const int64_t r = (group << (5 - w.lg)) + (lane >> w.lg);
+        if (r < w.rows)
+            for (int x = xl; x < end; x += 32) f(r, first + x);
+    }
+}
+
+template <typename S, typename R>
+__global__ void __launch_bounds__(kTpb) k_monitor(Lat<S, R> L, RowWalk w, Mask mk, Reduce red, double* out) {
+    double s[5] = {0, 0, 0, 0, 0};
+    walk_rows(w, [&](int64_t r, int x) {
+        if (mk.bits != nullptr && (mk.bits[r * mk.wpr + (x >> 5)] >> (x & 31)) & 1u) {
+            s[0] += 1.0;
+            return;
         }
+        double rho, xj, yj, zj, usq;
+        node_sums(L, r * w.l + x, rho, xj, yj, zj, usq);
+        s[0] += rho; s[1] += xj; s[2] += yj; s[3] += zj; s[4] += usq;
+    });
     block_reduce_store<5>(s, red, out);
 }
 
@@ -365,19 +378,16 @@ __global__ void __launch_bounds__(kTpb) k_monitor(Lat<S, R> L, int l, int64_t ro
 // a probe box, ...): {count, sum rho, sum ux, sum uy, sum uz, sum u^2}, u = j/rho
 // as CODE/SRC/diagno.F90:86-105 computes it.
 template <typename S, typename R>
-__global__ void __launch_bounds__(kTpb) k_region_sums(Lat<S, R> L, int l, int64_t rows, Mask mk, const uint8_t* region,
+__global__ void __launch_bounds__(kTpb) k_region_sums(Lat<S, R> L, RowWalk w, Mask mk, const uint8_t* region,
                                                       Reduce red, double* out) {
     double s[6] = {0, 0, 0, 0, 0, 0};
-    const int lane = threadIdx.x & 31;
-    const int64_t step = (int64_t)gridDim.x * (kTpb / 32);
-    for (int64_t r = (int64_t)blockIdx.x * (kTpb / 32) + (threadIdx.x >> 5); r < rows; r += step)
-        for (int x = lane; x < l; x += 32) {
-            if (!region[r * l + x]) continue;
-            if (mk.bits != nullptr && (mk.bits[r * mk.wpr + (x >> 5)] >> lane) & 1u) continue;
-            double rho, xj, yj, zj, usq;
-            node_sums(L, r * l + x, rho, xj, yj, zj, usq);
-            s[0] += 1.0; s[1] += rho; s[2] += xj; s[3] += yj; s[4] += zj; s[5] += usq;
-        }
+    walk_rows(w, [&](int64_t r, int x) {
+        if (!region[r * w.l + x]) return;
+        if (mk.bits != nullptr && (mk.bits[r * mk.wpr + (x >> 5)] >> (x & 31)) & 1u) return;
+        double rho, xj, yj, zj, usq;
+        node_sums(L, r * w.l + x, rho, xj, yj, zj, usq);
+        s[0] += 1.0; s[1] += rho; s[2] += xj; s[3] += yj; s[4] += zj; s[5] += usq;
+    });
     block_reduce_store<6>(s, red, out);
 }
 
@@ -425,33 +435,33 @@ __global__ void k_line(Lat<S, R> L, Geo g, int axis, int c1, int c2, double* out
 }
 
 // Plane means (CODE/SRC/varm.F90:42-98 for axis z): FP64 sums of u, w, v (momentum times 1/den
-// in R) and den over the nodes of each plane, divided by their number, in two passes with a
-// fixed order.  A thread keeps its x and walks rows, so the state is read once and coalesced
+// in R) and den over the nodes of each plane, divided by their number, in two passes (one for small
+// planes, row_walk.h) with a fixed order.  A thread keeps its x and walks rows, so the state is read once and coalesced
 // for every axis: rows of one plane for the planes normal to y and z, with a sum over the block
 // at the end, and a share of all rows for those normal to x, where the thread's column is the
 // plane.  (One block per plane, walked by 256 threads, a row's stride apart for the planes
 // normal to x, took 1110 / 848 / 803 us for the planes normal to x / y / z at 384x192x192 FP32
 // and 27.9 / 6.2 / 5.8 ms at 1024x512x512 FP16; now 200 us and 2.6..3.5 ms.  A warp per row
 // with a sum over its lanes at the end of each: 226 us, 3.5 ms.)
-struct PlaneWalk {
-    int l, rows;          // rows of a plane (all rows for axis 0)
-    int shares, xblocks;  // thread blocks a plane is dealt to, by rows and along x
-    int64_t plane, row;   // row index of row t of plane p: p * plane + t * row
-};
-
 template <typename S, typename R, bool COLUMN>
-__global__ void __launch_bounds__(128) k_plane_sums(Lat<S, R> L, PlaneWalk w, double* part) {
+__global__ void __launch_bounds__(128) k_plane_sums(Lat<S, R> L, PlaneWalk w, double cnt, double* part) {
     const int xb = blockIdx.x % w.xblocks, ps = blockIdx.x / w.xblocks;  // ps = plane * shares + share
     const int share = ps % w.shares;
     const int64_t first = (int64_t)(ps / w.shares) * w.plane;
     const int x = xb * blockDim.x + threadIdx.x;
     double s[4] = {0, 0, 0, 0};
-    if (x < w.l)
+    auto column = [&](int64_t xi) {
         for (int t = share * blockDim.y + threadIdx.y; t < w.rows; t += w.shares * blockDim.y) {
             R den, u, v, z;
-            ref_macro(L, (first + t * w.row) * w.l + x, false, den, u, v, z);
+            ref_macro(L, (first + t * w.row) * w.l + xi, false, den, u, v, z);
             s[0] += (double)u; s[1] += (double)v; s[2] += (double)z; s[3] += (double)den;
         }
+    };
+    if constexpr (COLUMN) {
+        if (x < w.l) column(x);
+    } else {
+        for (int64_t xi = x; xi < w.l; xi += (int64_t)w.xblocks * blockDim.x) column(xi);
+    }
     if constexpr (COLUMN) {  // part[((share * blockDim.y + threadIdx.y) * 4 + c) * l + x]
         if (x < w.l)
 #pragma unroll
@@ -466,7 +476,8 @@ __global__ void __launch_bounds__(128) k_plane_sums(Lat<S, R> L, PlaneWalk w, do
 #pragma unroll
             for (int c = 0; c < 4; ++c) sh[tid >> 5][c] = s[c];
         __syncthreads();
-        if (tid < 4) part[4 * (int64_t)blockIdx.x + tid] = (sh[0][tid] + sh[1][tid]) + (sh[2][tid] + sh[3][tid]);
+        if (tid < 4)  // cnt: nodes of the plane, where this block has all of them
+            part[4 * (int64_t)blockIdx.x + tid] = ((sh[0][tid] + sh[1][tid]) + (sh[2][tid] + sh[3][tid])) / cnt;
     }
 }
 
@@ -878,16 +889,16 @@ void launch_fill_xface(const Lat<S, R>& L, const Geo& g, cudaStream_t st) {
 template <typename S, typename R>
 void launch_monitor(const Lat<S, R>& L, const Geo& g, const Mask& mk, const Reduce& red, double* out,
                     cudaStream_t st) {
-    const int64_t rows = (int64_t)g.m * g.n;
-    k_monitor<S, R><<<grid_for(rows, kTpb / 32, (unsigned)red.max_blocks), kTpb, 0, st>>>(L, g.l, rows, mk, red, out);
+    const RowWalk w = row_walk(g.l, (int64_t)g.m * g.n);
+    k_monitor<S, R><<<grid_for(w.units, kTpb / 32, (unsigned)red.max_blocks), kTpb, 0, st>>>(L, w, mk, red, out);
 }
 
 template <typename S, typename R>
 void launch_region_sums(const Lat<S, R>& L, const Geo& g, const Mask& mk, const uint8_t* region, const Reduce& red,
                         double* out, cudaStream_t st) {
-    const int64_t rows = (int64_t)g.m * g.n;
-    k_region_sums<S, R><<<grid_for(rows, kTpb / 32, (unsigned)red.max_blocks), kTpb, 0, st>>>(L, g.l, rows, mk, region,
-                                                                                             red, out);
+    const RowWalk w = row_walk(g.l, (int64_t)g.m * g.n);
+    k_region_sums<S, R><<<grid_for(w.units, kTpb / 32, (unsigned)red.max_blocks), kTpb, 0, st>>>(L, w, mk, region, red,
+                                                                                                out);
 }
 
 template <typename S, typename R>
@@ -896,46 +907,24 @@ void launch_line(const Lat<S, R>& L, const Geo& g, int axis, int c1, int c2, dou
     k_line<S, R><<<(len + 127) / 128, 128, 0, st>>>(L, g, axis, c1, c2, out);
 }
 
-// Blocks of 128 threads: as many along x as a row fills, the rest over rows; enough shares for
-// a few waves of the 12 blocks an SM holds, but eight rows a thread at least, so that the
-// partial sums stay below the size of the staging buffer they go to.
-static PlaneWalk plane_walk(const Geo& g, int axis, dim3* block, int* planes) {
-    PlaneWalk w;
-    const int tx = g.l > 64 ? 128 : (g.l > 32 ? 64 : 32);
-    *block = dim3(tx, 128 / tx);
-    *planes = axis == 0 ? 1 : (axis == 1 ? g.m : g.n);
-    w.l = g.l;
-    w.rows = axis == 0 ? g.m * g.n : (axis == 1 ? g.n : g.m);
-    w.xblocks = (g.l + tx - 1) / tx;
-    w.plane = axis == 1 ? 1 : g.m;
-    w.row = axis == 1 ? g.m : 1;
-    const int64_t most = w.rows / (8 * (int)block->y);
-    const int64_t want = 148 * 12 * (axis == 0 ? 1 : 3) / ((int64_t)*planes * w.xblocks);
-    w.shares = (int)std::max<int64_t>(1, std::min(most, want));
-    return w;
-}
-
-int64_t plane_means_scratch(const Geo& g, int axis) {
-    dim3 block;
-    int planes;
-    const PlaneWalk w = plane_walk(g, axis, &block, &planes);
-    return 4 * (axis == 0 ? (int64_t)w.shares * block.y * g.l : (int64_t)planes * w.shares * w.xblocks);
-}
+int64_t plane_means_scratch(const Geo& g, int axis) { return plane_split(g.l, g.m, g.n, axis).scratch(axis); }
 
 template <typename S, typename R>
 void launch_plane_means(const Lat<S, R>& L, const Geo& g, int axis, double* out, double* scratch, cudaStream_t st) {
-    dim3 block;
-    int planes;
-    const PlaneWalk w = plane_walk(g, axis, &block, &planes);
-    const unsigned blocks = (unsigned)(planes * w.shares * w.xblocks);
+    const PlaneSplit p = plane_split(g.l, g.m, g.n, axis);
+    const PlaneWalk& w = p.w;
+    const dim3 block(p.tx, p.ty);
+    const unsigned blocks = (unsigned)p.blocks();
+    const int parts = w.shares * w.xblocks;
+    const double nodes = axis == 0 ? (double)g.m * g.n : (double)g.l * w.rows;
     if (axis == 0) {
-        k_plane_sums<S, R, true><<<blocks, block, 0, st>>>(L, w, scratch);
-        k_add_planes<<<g.l, 256, 0, st>>>(scratch, 1, g.l, 4 * (int64_t)g.l, w.shares * (int)block.y,
-                                          (double)g.m * g.n, out);
+        k_plane_sums<S, R, true><<<blocks, block, 0, st>>>(L, w, 1.0, scratch);
+        k_add_planes<<<g.l, 256, 0, st>>>(scratch, 1, g.l, 4 * (int64_t)g.l, w.shares * p.ty, nodes, out);
+    } else if (parts == 1) {
+        k_plane_sums<S, R, false><<<blocks, block, 0, st>>>(L, w, nodes, out);
     } else {
-        k_plane_sums<S, R, false><<<blocks, block, 0, st>>>(L, w, scratch);
-        const int parts = w.shares * w.xblocks;
-        k_add_planes<<<planes, 256, 0, st>>>(scratch, 4 * (int64_t)parts, 1, 4, parts, (double)g.l * w.rows, out);
+        k_plane_sums<S, R, false><<<blocks, block, 0, st>>>(L, w, 1.0, scratch);
+        k_add_planes<<<p.planes, 256, 0, st>>>(scratch, 4 * (int64_t)parts, 1, 4, parts, nodes, out);
     }
 }
 
