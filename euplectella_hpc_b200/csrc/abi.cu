@@ -716,13 +716,15 @@ int install_mask(eup_handle* h, uint32_t* bits, int wpr, int64_t nsolid) {
     int64_t nblist = 0;
     LinksDevice links;
     if (nsolid > 0) {
-        // flags, link words and compaction scratch share the staging buffer, which the next
-        // state transfer of this precision needs at its full size anyway
+        // flags, link words and compaction scratch share the staging buffer.  Below 1 MB it grows no
+        // further than they need: an allocation of a megabyte takes 0.4 ms and its release 0.3, a
+        // smaller one microseconds.  Beyond, it is made as large at once as the next state
+        // transfer of this precision needs it.
         const size_t flags_bytes = ((size_t)g.N + 255) / 256 * 256;
         const size_t words_bytes = (sizeof(uint64_t) * (size_t)nsolid + 255) / 256 * 256;
         const size_t pop = (size_t)(g.l + 2) * (g.m + 2) * (g.n + 2) * (h->prec == EUP_FP64 ? 8 : 4);
-        const size_t want = std::max(flags_bytes + words_bytes + ((size_t)1 << 16),
-                                     Q * pop <= kBatchBytes ? Q * pop : pop);
+        size_t want = flags_bytes + words_bytes + ((size_t)1 << 16);
+        if (want >= (size_t)1 << 20) want = std::max(want, Q * pop <= kBatchBytes ? Q * pop : pop);
         const int rc = ensure_staging(h, want);
         if (rc) {
             cudaFree(bits);

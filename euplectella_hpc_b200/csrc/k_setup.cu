@@ -182,6 +182,7 @@ cudaError_t compact_links(At at, int64_t n, int64_t count, Link* out, void* buf,
         if (e == cudaSuccess) e = tmp.get(buf, have, 256 + bytes);
         if (e == cudaSuccess)
             e = cub::DeviceSelect::If(tmp.p + 256, bytes, in, out + done, (int*)tmp.p, items, IsLink(), st);
+        if (per >= 18) return e;  // all of them at once: `count` items are there
         if (e == cudaSuccess) e = cudaMemcpyAsync(&got, tmp.p, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         done += got;
@@ -334,6 +335,8 @@ cudaError_t build_links(const Geo& g, const int bc[6], const int32_t* list, cons
     const LinkAt at{g, list, words, n, 0, bc[0] == 0 && bc[1] == 0, bc[2] == 0 && bc[3] == 0, bc[4] == 0 && bc[5] == 0};
     if (e == cudaSuccess) e = compact_links(FluidLinkAt{at}, n, (int64_t)cnt[0], fluid, scratch, scratch_bytes, st);
     if (e == cudaSuccess) e = compact_links(HaloLinkAt{at}, n, (int64_t)cnt[1], halo, scratch, scratch_bytes, st);
+    const cudaError_t es = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) {
         if (fluid) cudaFree(fluid);
         if (halo) cudaFree(halo);
