@@ -173,8 +173,8 @@ Mask make_mask(const eup_handle* h) { return Mask{h->bits, h->wpr}; }
 // EUP_STEP_VARIANT without bit 12: one launch per halo block instead of one for all.
 bool bc_separate(const eup_handle* h) { return !(h->variant & 4096); }
 
-bool pbb_one_pass(const eup_handle* h, int64_t sectors, bool force) {
-    return pbb_in_one_pass(h->g.l, h->g.N, h->sbytes, h->variant, sectors, force, kReduceMaxBlocks);
+bool pbb_one_pass(const eup_handle* h, int64_t sectors, int64_t voxels, bool force) {
+    return pbb_in_one_pass(h->g.l, h->g.N, h->sbytes, h->variant, sectors, voxels, force, kReduceMaxBlocks);
 }
 
 Reduce make_reduce(const eup_handle* h) { return Reduce{h->partials, h->counter, kReduceMaxBlocks}; }
@@ -1831,8 +1831,8 @@ int eup_set_solid_fraction(eup_handle* h, const double* ns) {
             sectors += list.empty() || list.back() / 8 != t / 8;
             list.push_back((int32_t)t);
         }
-    h->ns_whole = pbb_one_pass(h, sectors, true);
-    h->ns_again = pbb_one_pass(h, sectors, false);
+    h->ns_whole = pbb_one_pass(h, sectors, (int64_t)list.size(), true);
+    h->ns_again = pbb_one_pass(h, sectors, (int64_t)list.size(), false);
     if (!h->ns) CK(h, cudaMalloc(&h->ns, h->rbytes * N));
     if (h->ns_list) cudaFree(h->ns_list);
     h->ns_list = nullptr;
