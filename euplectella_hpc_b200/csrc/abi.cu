@@ -479,12 +479,15 @@ int end_transfer(eup_handle* h, cudaError_t e, const char* who) {
     return e == cudaSuccess ? EUP_OK : cuda_fail(h, e, who);
 }
 
-// A whole state of at most this many bytes crosses in one piece: one launch for the 19 populations
-// and, where the caller's arrays lie one behind the other, one copy.  Population by population,
-// the copies beside the launches / in one piece, up and down, page-locked: 1.7 MB 181+143 / 84+57 us,
-// 12.5 MB 402+309 / 297+265, 32.6 MB 754+669 / 693+650, 95 MB 1877+1832 / 1922+1860, where the launches
-// are hidden and the copy alone counts.
-constexpr size_t kBatchBytes = (size_t)48 << 20;
+// A whole state of at most kBatchBytes crosses in one piece: one launch for the 19 populations and,
+// where the caller's arrays lie one behind the other, one copy.  Page-locked arrays that lie apart
+// take nineteen copies either way, and beyond kApartBytes those are better beside the launches.
+// Up + down in us, population by population / in one piece, FP32: one page-locked array
+// 1.7 MB 201+136 / 85+56, 12 MB 598+296 / 314+251, 27 MB 636+576 / 709+553, 40 MB 881+787 / 1042+780 (the
+// uploads scatter by a factor of two); page-locked arrays apart 1.7 MB 192+125 / 163+116, 8 MB
+// 291+235 / 284+239, 16 MB 475+362 / 565+389, 27 MB 624+577 / 779+611; pageable arrays apart 1.7 MB
+// 234+476 / 204+379, 27 MB 1551+2288 / 1583+2124.
+constexpr size_t kBatchBytes = (size_t)48 << 20, kApartBytes = (size_t)8 << 20;
 
 bool one_behind_the_other(const void* const pops[19], size_t bytes) {
     for (int q = 1; q < Q; ++q)
@@ -510,6 +513,14 @@ cudaError_t copy_populations(char* dev, void* const host[19], size_t bytes, bool
     cudaError_t e = cudaSuccess;
     for (int q = 0; q < Q && e == cudaSuccess; ++q) e = copy(q, bytes);
     return e;
+}
+
+bool in_one_piece(const void* const pops[19], size_t bytes) {
+    if (Q * bytes > kBatchBytes) return false;
+    if (Q * bytes <= kApartBytes || one_behind_the_other(pops, bytes)) return true;
+    cudaPointerAttributes at = {};
+    if (cudaPointerGetAttributes(&at, pops[0]) != cudaSuccess) cudaGetLastError();
+    return at.type == cudaMemoryTypeUnregistered;
 }
 
 int ensure_staging(eup_handle* h, size_t bytes) {
@@ -910,7 +921,7 @@ int eup_upload(eup_handle* h, const void* const pops[19], int32_t elem_bytes, in
         if (!pops[q]) return fail(h, EUP_ERR_INVALID_ARG, "eup_upload: null population array");
     const Geo& g = h->g;
     const size_t bytes = (size_t)(g.l + 2) * (g.m + 2) * (g.n + 2) * elem_bytes;
-    if (Q * bytes <= kBatchBytes) {
+    if (in_one_piece(pops, bytes)) {
         if ((rc = ensure_staging(h, Q * bytes)) || (rc = begin_upload_check(h))) return rc;
         char* buf = static_cast<char*>(h->staging);
         cudaError_t e = copy_populations(buf, const_cast<void* const*>(pops), bytes, true, h->stream);
@@ -1042,7 +1053,7 @@ int eup_download(eup_handle* h, void* const pops[19], int32_t elem_bytes) {
         if (!pops[q]) return fail(h, EUP_ERR_INVALID_ARG, "eup_download: null population array");
     const Geo& g = h->g;
     const size_t bytes = (size_t)(g.l + 2) * (g.m + 2) * (g.n + 2) * elem_bytes;
-    if (Q * bytes <= kBatchBytes) {
+    if (in_one_piece(pops, bytes)) {
         if ((rc = ensure_staging(h, Q * bytes))) return rc;
         char* buf = static_cast<char*>(h->staging);
         DISPATCH(h, download_q, h, 0, Q, elem_bytes, buf);

@@ -75,3 +75,25 @@ def test_separate_page_locked_arrays(eup, require_gpu):
         s.upload_ptrs([x.data_ptr() for x in up], 4)
         s.download_ptrs([x.data_ptr() for x in down], 4)
     assert np.array_equal(np.stack([x.numpy() for x in down]), start)
+
+
+@pytest.mark.parametrize("size", [(70, 50, 24), (96, 48, 40)], ids=["7MB", "16MB"])
+@pytest.mark.parametrize("locked", [True, False], ids=["page-locked", "pageable"])
+def test_arrays_apart(eup, require_gpu, size, locked):
+    """Both sides of the size from which page-locked arrays apart cross population by population."""
+    import torch
+    l, m, n = size
+    start = eup.init_equilibrium(l, m, n, 0.05, 1e-3, 21, np.float32)
+    count = start[0].size
+
+    def arrays():
+        t = [torch.zeros(count + 4096, pin_memory=locked) for _ in range(19)]  # gaps between them
+        return t, [x.numpy()[:count].reshape(start[0].shape) for x in t]
+
+    (keep_up, up), (keep_down, down) = arrays(), arrays()
+    for q in range(19):
+        up[q][...] = start[q]
+    with eup.Solver(eup.Config(l, m, n, svisc=0.05, u_inflow=0.05)) as s:
+        s.upload_ptrs([x.ctypes.data for x in up], 4)
+        s.download_ptrs([x.ctypes.data for x in down], 4)
+    assert np.array_equal(np.stack(down), start)
