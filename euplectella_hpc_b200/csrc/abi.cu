@@ -655,13 +655,7 @@ int eup_create(const eup_config* cfg, eup_handle** out) {
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(x-face copy)"));
     cudaMemsetAsync(h->xface, 0, xface_bytes, h->stream);
     const HaloEdges edges = build_halo_edges(h->g, cfg->bc);
-    HaloEdge* d_edges = nullptr;
-    if ((e = cudaMalloc(&d_edges, sizeof(HaloEdge) * (edges.e.size() + 1))) != cudaSuccess)
-        return cleanup_fail(cuda_fail(h, e, "cudaMalloc(halo edges)"));
-    h->edges.e = d_edges;
-    for (int b = 0; b < 9; ++b) h->edges.first[b] = edges.first[b];
-    if ((e = cudaMemcpyAsync(d_edges, edges.e.data(), sizeof(HaloEdge) * edges.e.size(), cudaMemcpyHostToDevice,
-                             h->stream)) != cudaSuccess)
+    if ((e = put_halo_edges(edges, &h->edges, h->stream)) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "halo edges"));
     if ((e = cudaMalloc(&h->d_itime, sizeof(int64_t))) != cudaSuccess)
         return cleanup_fail(cuda_fail(h, e, "cudaMalloc(step counter)"));

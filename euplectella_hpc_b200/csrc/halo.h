@@ -15,7 +15,7 @@
 //    read and passed on by the very item that replaces them.
 //
 // So the items give the reference's halo in any order (tests run them in random order against
-// the oracle).  They are host code: the device runs them in the form halo_plan.cpp records,
+// the oracle).  They are host code: the device runs them in the form halo_plan.cu records,
 // five strided copies per face and a table for the edge lines.
 // q is the reference's population number, 1..18.
 #pragma once

@@ -1,6 +1,10 @@
 // The halo items of halo.h in the form k_halo runs: per face five strided copies (outflow
 // equilibria, constants), recorded from one item in the middle of the face, and a table of
-// what lands on the twelve edge lines, recorded from every item that can reach them.  Host code.
+// what lands on the twelve edge lines, recorded on the host from the items near the ends of the
+// lines and one between, which repeats along the line, and written out on the device.
+#include <algorithm>
+#include <utility>
+
 #include "halo.h"
 #include "internal.h"
 
@@ -55,53 +59,137 @@ struct Recorder {
 
 }  // namespace
 
-HaloEdges build_halo_edges(const Geo& g, const int bc[6]) {
+namespace {
+
+HaloEdge edge_of(const Geo& g, const Store_& s) {
+    HaloEdge e;
+    e.dst = (int64_t)(s.q - 1) * g.G + g.gidx(s.i, s.j, s.k);
+    e.q = s.v.q - 1;
+    switch (s.v.kind) {
+        case Sym::kCopy:
+            e.kind = s.v.lid == 0 ? kEdgeCopy : (s.v.lid > 0 ? kEdgeCopyPlus : kEdgeCopyMinus);
+            e.src = g.lin(s.v.i, s.v.j, s.v.k);
+            break;
+        case Sym::kOld:
+            e.kind = kEdgeOld;
+            e.src = (int64_t)(s.v.q - 1) * g.G + g.gidx(s.v.i, s.v.j, s.v.k);
+            break;
+        case Sym::kOutflow:
+            e.kind = kEdgeOutflow;
+            e.q = s.v.q;
+            e.src = (int64_t)(s.v.j - 1) + (int64_t)(s.v.k - 1) * g.m;
+            break;
+        default:
+            e.kind = kEdgeConst;
+            e.q = s.v.q;
+            e.src = 0;
+    }
+    return e;
+}
+
+// The coordinates lo .. lo+count-1 as runs (first, length): one by one within four of a place where
+// an item's conditions change, else as long as possible.  An item reads and writes within one node of
+// its own coordinates, so the items of a run differ by a shift alone.
+std::vector<std::pair<int, int>> runs_along(int lo, int count, std::vector<int> changes, bool one_by_one) {
+    changes.push_back(lo);
+    changes.push_back(lo + count - 1);
+    std::vector<std::pair<int, int>> out;
+    for (int64_t c = lo; c < (int64_t)lo + count;) {
+        int64_t next = (int64_t)lo + count;
+        bool near = one_by_one;
+        for (const int64_t p : changes) {
+            near |= c >= p - 4 && c <= p + 4;
+            if (p - 4 > c) next = std::min(next, p - 4);
+        }
+        const int64_t length = near ? 1 : next - c;
+        out.push_back({(int)c, (int)length});
+        c += length;
+    }
+    return out;
+}
+
+// Thread t writes edge t: the last run that starts at or before it, shifted.
+__global__ void k_fill_edges(const HaloEdgeRun* runs, int nruns, int64_t total, HaloEdge* out) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    int lo = 0, hi = nruns;  // runs[lo].at <= t < runs[hi].at
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) / 2;
+        if (runs[mid].at <= t) lo = mid;
+        else hi = mid;
+    }
+    const HaloEdgeRun r = runs[lo];
+    HaloEdge e = r.e;
+    e.dst += (t - r.at) * r.dst_step;
+    e.src += (t - r.at) * r.src_step;
+    out[t] = e;
+}
+
+}  // namespace
+
+HaloEdges build_halo_edges(const Geo& g, const int bc[6], bool one_by_one) {
     HaloEdges out;
-    std::vector<Store_> st;
+    std::vector<Store_> st, after;
     Recorder rec{HaloConf(g.l, g.m, g.n, bc), 0, true, &st};
     const HaloConf& c = rec.c;
+    int64_t at = 0;
+    // item (ia, ib) and the `length - 1` behind it along a (or b)
+    auto record = [&](int b, int ia, int ib, int length, bool along_a) {
+        st.clear();
+        halo_item(rec, b, ia, ib);
+        if (length > 1) {
+            after.swap(st);
+            st.clear();
+            halo_item(rec, b, ia + along_a, ib + !along_a);
+            after.swap(st);
+        }
+        for (size_t t = 0; t < st.size(); ++t) {
+            HaloEdgeRun r{edge_of(g, st[t]), 0, 0, at};
+            if (length > 1) {
+                const HaloEdge next = edge_of(g, after[t]);
+                r.dst_step = next.dst - r.e.dst;
+                r.src_step = next.src - r.e.src;
+            }
+            out.runs.push_back(r);
+            at += length;
+        }
+    };
     for (int b = 0; b < kHaloBlocks; ++b) {
         rec.block = b;
-        out.first[b] = (int64_t)out.e.size();
+        out.first[b] = at;
         const HaloRange r = halo_range(c, b);
+        if (r.size() == 0) continue;
+        // an item reaches an edge line only from the outermost rows and columns of its range
         const bool all = b == kHaloFrontFix || b == kHaloEdgeFix;
-        st.clear();
-        for (int y = 0; y < r.nb; ++y) {
-            // an item reaches an edge line only from the outermost rows and columns of its range
-            const bool row = all || y == 0 || y == r.nb - 1;
-            for (int x = 0; x < r.na; ++x) {
-                if (!row && x > 0) x = r.na - 1;
-                halo_item(rec, b, r.a0 + x, r.b0 + y);
+        const auto xs = runs_along(r.a0, r.na, b == kHaloFrontFix ? std::vector<int>{c.m, c.n} : std::vector<int>{},
+                                   one_by_one);
+        for (const auto& y : runs_along(r.b0, r.nb, {}, one_by_one)) {
+            if (all || y.first == r.b0 || y.first == r.b0 + r.nb - 1) {
+                for (const auto& x : xs) record(b, x.first, y.first, x.second, true);
+            } else {
+                record(b, r.a0, y.first, y.second, false);
+                if (r.na > 1) record(b, r.a0 + r.na - 1, y.first, y.second, false);
             }
-        }
-        for (const Store_& s : st) {
-            HaloEdge e;
-            e.dst = (int64_t)(s.q - 1) * g.G + g.gidx(s.i, s.j, s.k);
-            e.q = s.v.q - 1;
-            switch (s.v.kind) {
-                case Sym::kCopy:
-                    e.kind = s.v.lid == 0 ? kEdgeCopy : (s.v.lid > 0 ? kEdgeCopyPlus : kEdgeCopyMinus);
-                    e.src = g.lin(s.v.i, s.v.j, s.v.k);
-                    break;
-                case Sym::kOld:
-                    e.kind = kEdgeOld;
-                    e.src = (int64_t)(s.v.q - 1) * g.G + g.gidx(s.v.i, s.v.j, s.v.k);
-                    break;
-                case Sym::kOutflow:
-                    e.kind = kEdgeOutflow;
-                    e.q = s.v.q;
-                    e.src = (int64_t)(s.v.j - 1) + (int64_t)(s.v.k - 1) * g.m;
-                    break;
-                default:
-                    e.kind = kEdgeConst;
-                    e.q = s.v.q;
-                    e.src = 0;
-            }
-            out.e.push_back(e);
         }
     }
-    out.first[kHaloBlocks] = (int64_t)out.e.size();
+    out.first[kHaloBlocks] = at;
     return out;
+}
+
+cudaError_t put_halo_edges(const HaloEdges& edges, HaloEdgesDevice* out, cudaStream_t st) {
+    const int64_t total = edges.first[kHaloBlocks];
+    char* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, sizeof(HaloEdge) * total + sizeof(HaloEdgeRun) * edges.runs.size() + 1);
+    if (e != cudaSuccess) return e;
+    out->e = reinterpret_cast<HaloEdge*>(mem);  // the runs behind the table
+    for (int b = 0; b <= kHaloBlocks; ++b) out->first[b] = edges.first[b];
+    if (total == 0) return cudaSuccess;
+    HaloEdgeRun* runs = reinterpret_cast<HaloEdgeRun*>(mem + sizeof(HaloEdge) * total);
+    e = cudaMemcpyAsync(runs, edges.runs.data(), sizeof(HaloEdgeRun) * edges.runs.size(), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return e;
+    k_fill_edges<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(runs, (int)edges.runs.size(), total,
+                                                                  reinterpret_cast<HaloEdge*>(mem));
+    return cudaGetLastError();
 }
 
 HaloFace record_halo_face(const Geo& g, const int bc[6], int b) {
@@ -159,3 +247,28 @@ HaloFace record_halo_face(const Geo& g, const int bc[6], int b) {
 }
 
 }  // namespace eup
+
+// The edge table on the host, for tests: `out` takes (dst, src, q, kind, block) of each store, at most
+// `cap` of them; the items recorded one by one, or as runs.  Returns how many there are.
+extern "C" int64_t eup_internal_halo_edges(int l, int m, int n, const int* bc, int one_by_one, int64_t* out, int64_t cap) {
+    using namespace eup;
+    Geo g{};
+    g.init(l, m, n);
+    const HaloEdges e = build_halo_edges(g, bc, one_by_one != 0);
+    const int64_t total = e.first[kHaloBlocks];
+    for (size_t r = 0; r < e.runs.size(); ++r) {
+        const HaloEdgeRun& run = e.runs[r];
+        const int64_t end = r + 1 < e.runs.size() ? e.runs[r + 1].at : total;
+        int block = 0;
+        while (run.at >= e.first[block + 1]) ++block;
+        for (int64_t t = run.at; t < end && t < cap; ++t) {
+            int64_t* o = out + 5 * t;
+            o[0] = run.e.dst + (t - run.at) * run.dst_step;
+            o[1] = run.e.src + (t - run.at) * run.src_step;
+            o[2] = run.e.q;
+            o[3] = run.e.kind;
+            o[4] = block;
+        }
+    }
+    return total;
+}
