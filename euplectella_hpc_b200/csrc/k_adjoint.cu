@@ -64,12 +64,6 @@ struct PState {
     }
 };
 
-template <typename R>
-__device__ __forceinline__ R pull_pre(const Lat<R, R>& L, const Geo& g, int q, int i, int j, int k, int64_t lin,
-                                      bool face) {
-    return PState<R, R>::pull_f(L, g, q, i, j, k, lin, face);
-}
-
 // The partial-bounce-back step in two passes is the plain stream-collide (every node's BGK value, the
 // same kernels and bits as the plain step) followed by this kernel over the list of
 // voxels with n_s > 0: it pulls their pre-collision populations again, mixes

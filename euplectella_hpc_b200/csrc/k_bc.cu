@@ -1,8 +1,9 @@
-// Boundary side of the time step: halo planes (CODE/SRC/bcond.bc.F90),
+// Boundary side of the time step: halo planes (CODE/SRC/bcond.bc.F90) and
 // bounce-back on solid voxels with the momentum-exchange force
-// (CODE/SRC/bcond.obs.F90), the FP64 monitor (CODE/SRC/diagno.F90), probes
-// (CODE/SRC/probe_global.F90) and the host-layout scatter/gather used by
-// upload and download.  All of it is O(surface) or O(solid surface) work.
+// (CODE/SRC/bcond.obs.F90), O(surface) and O(solid surface) work; the diagnostics,
+// some of a few nodes (CODE/SRC/probe_global.F90, lines, control volume), some of all of
+// them (the FP64 monitor of CODE/SRC/diagno.F90, region sums, plane means); and the
+// host-layout scatter/gather of upload and download, which move the whole state.
 #include "init_eq.h"
 #include <algorithm>
 
@@ -134,6 +135,9 @@ __device__ __forceinline__ void sum_partials(const ForceSum& a, bool advance) {
     if (advance && threadIdx.x == 0) *a.d_itime = t + 1;
 }
 
+// Where the links are many the loads in flight count: with 20 % of the voxels solid at random,
+// 256x128x64 FP16, a step takes 81.9 us with 32 registers (16-bit storage spills one of them once) and
+// 86.1 with 36; FP64's six sums take 40, and 214 us for 210 with three plain sums.
 template <typename S, typename R>
 __global__ void __launch_bounds__(kTpb, sizeof(R) == 8 ? 6 : 8) k_bounce(const __grid_constant__ BounceArgs<S, R> p) {
     chain_open();

@@ -284,16 +284,6 @@ __device__ __forceinline__ R bc_load(const Lat<S, R>& L, const Geo& g, int q, in
     return lat_load(L, g, q, i, j, k);
 }
 
-// Value a later lattice load returns for an arithmetic value v of population q.
-template <typename S, typename R>
-__device__ __forceinline__ R stored_value(R v, int q, R scale, R inv_scale) {
-    return Store<S, R>::load(Store<S, R>::store(v, q, scale), q, inv_scale);
-}
-template <typename S, typename R>
-__device__ __forceinline__ void ghost_store(const Lat<S, R>& L, const Geo& g, int q, int i, int j, int k, R v) {
-    L.ghost[(int64_t)q * g.G + g.gidx(i, j, k)] = v;
-}
-
 // ---------------------------------------------------------------------------
 // BGK collision of one node, CODE/SRC/col.F90:127-229, same operation order.
 // x[0..17] are the streamed populations b01..b18, x[18] is a19; on return x
