@@ -108,20 +108,21 @@ std::vector<std::pair<int, int>> runs_along(int lo, int count, std::vector<int> 
     return out;
 }
 
-// Thread t writes edge t: the last run that starts at or before it, shifted.
+// Thread t writes edge t: it lies in the group of the last run that starts at or before it.
 __global__ void k_fill_edges(const HaloEdgeRun* runs, int nruns, int64_t total, HaloEdge* out) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    int lo = 0, hi = nruns;  // runs[lo].at <= t < runs[hi].at
+    int lo = 0, hi = nruns;  // runs[lo].at <= t, and runs[hi].at > t or hi = nruns
     while (hi - lo > 1) {
         const int mid = (lo + hi) / 2;
         if (runs[mid].at <= t) lo = mid;
         else hi = mid;
     }
-    const HaloEdgeRun r = runs[lo];
+    const int64_t u = t - runs[lo].at, along = u / runs[lo].stores;
+    const HaloEdgeRun r = runs[lo - (runs[lo].stores - 1) + (int)(u - along * runs[lo].stores)];
     HaloEdge e = r.e;
-    e.dst += (t - r.at) * r.dst_step;
-    e.src += (t - r.at) * r.src_step;
+    e.dst += along * r.dst_step;
+    e.src += along * r.src_step;
     out[t] = e;
 }
 
@@ -129,30 +130,31 @@ __global__ void k_fill_edges(const HaloEdgeRun* runs, int nruns, int64_t total, 
 
 HaloEdges build_halo_edges(const Geo& g, const int bc[6], bool one_by_one) {
     HaloEdges out;
-    std::vector<Store_> st, after;
+    std::vector<Store_> st, one, next;
     Recorder rec{HaloConf(g.l, g.m, g.n, bc), 0, true, &st};
     const HaloConf& c = rec.c;
     int64_t at = 0;
-    // item (ia, ib) and the `length - 1` behind it along a (or b)
-    auto record = [&](int b, int ia, int ib, int length, bool along_a) {
-        st.clear();
-        halo_item(rec, b, ia, ib);
-        if (length > 1) {
-            after.swap(st);
+    // the stores of items (ia, ib) and, if it is another, (ia2, ib), and of the `length - 1` pairs
+    // behind them along a or b
+    auto record = [&](int b, int ia, int ia2, int ib, int length, bool along_a) {
+        auto items = [&](int d, std::vector<Store_>& to) {
             st.clear();
-            halo_item(rec, b, ia + along_a, ib + !along_a);
-            after.swap(st);
-        }
-        for (size_t t = 0; t < st.size(); ++t) {
-            HaloEdgeRun r{edge_of(g, st[t]), 0, 0, at};
+            halo_item(rec, b, ia + (along_a ? d : 0), ib + (along_a ? 0 : d));
+            if (ia2 != ia) halo_item(rec, b, ia2, ib + (along_a ? 0 : d));
+            to = st;
+        };
+        items(0, one);
+        if (length > 1) items(1, next);
+        for (size_t t = 0; t < one.size(); ++t) {
+            HaloEdgeRun r{edge_of(g, one[t]), 0, 0, at, (int32_t)one.size(), 0};
             if (length > 1) {
-                const HaloEdge next = edge_of(g, after[t]);
-                r.dst_step = next.dst - r.e.dst;
-                r.src_step = next.src - r.e.src;
+                const HaloEdge e = edge_of(g, next[t]);
+                r.dst_step = e.dst - r.e.dst;
+                r.src_step = e.src - r.e.src;
             }
             out.runs.push_back(r);
-            at += length;
         }
+        at += (int64_t)length * (int64_t)one.size();
     };
     for (int b = 0; b < kHaloBlocks; ++b) {
         rec.block = b;
@@ -165,10 +167,9 @@ HaloEdges build_halo_edges(const Geo& g, const int bc[6], bool one_by_one) {
                                    one_by_one);
         for (const auto& y : runs_along(r.b0, r.nb, {}, one_by_one)) {
             if (all || y.first == r.b0 || y.first == r.b0 + r.nb - 1) {
-                for (const auto& x : xs) record(b, x.first, y.first, x.second, true);
+                for (const auto& x : xs) record(b, x.first, x.first, y.first, x.second, true);
             } else {
-                record(b, r.a0, y.first, y.second, false);
-                if (r.na > 1) record(b, r.a0 + r.na - 1, y.first, y.second, false);
+                record(b, r.a0, r.a0 + r.na - 1, y.first, y.second, false);
             }
         }
     }
@@ -256,15 +257,16 @@ extern "C" int64_t eup_internal_halo_edges(int l, int m, int n, const int* bc, i
     g.init(l, m, n);
     const HaloEdges e = build_halo_edges(g, bc, one_by_one != 0);
     const int64_t total = e.first[kHaloBlocks];
-    for (size_t r = 0; r < e.runs.size(); ++r) {
-        const HaloEdgeRun& run = e.runs[r];
-        const int64_t end = r + 1 < e.runs.size() ? e.runs[r + 1].at : total;
+    for (size_t r = 0; r < e.runs.size(); r += e.runs[r].stores) {
+        const int stores = e.runs[r].stores;
+        const int64_t at = e.runs[r].at, end = r + stores < e.runs.size() ? e.runs[r + stores].at : total;
         int block = 0;
-        while (run.at >= e.first[block + 1]) ++block;
-        for (int64_t t = run.at; t < end && t < cap; ++t) {
+        while (at >= e.first[block + 1]) ++block;
+        for (int64_t t = at; t < end && t < cap; ++t) {
+            const HaloEdgeRun& run = e.runs[r + (t - at) % stores];
             int64_t* o = out + 5 * t;
-            o[0] = run.e.dst + (t - run.at) * run.dst_step;
-            o[1] = run.e.src + (t - run.at) * run.src_step;
+            o[0] = run.e.dst + (t - at) / stores * run.dst_step;
+            o[1] = run.e.src + (t - at) / stores * run.src_step;
             o[2] = run.e.q;
             o[3] = run.e.kind;
             o[4] = block;

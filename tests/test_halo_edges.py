@@ -27,10 +27,8 @@ def test_runs_equal_the_items(eup, size):
     longer = 0
     for bc in FLAGS:
         want, got = _edges(eup, size, bc, 1), _edges(eup, size, bc, 0)
-        assert want.shape == got.shape, bc
-        assert np.array_equal(np.unique(want, axis=0), np.unique(got, axis=0)), bc
+        assert np.array_equal(want, got), bc
         assert len(np.unique(want[:, 0])) == len(want), bc  # one store to a slot
-        assert np.array_equal(want[:, 4], got[:, 4]), bc  # blocks in their order
         longer += len(want)
     assert longer > 0
 
