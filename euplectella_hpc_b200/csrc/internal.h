@@ -150,8 +150,8 @@ struct HaloEdge {
 };
 // The edge stores of a step, grouped by the block that makes them (first[b] .. first[b + 1]): in
 // groups of `stores` runs that take turns from `at` on, each at a constant distance from its last.
-// (Run after run, the outflow stores of a column read its 18 x-face values once each and a step at
-// 256x128x64 FP16 takes 53.0 us for 52.0 with those of a row side by side.)  Recorded item by item
+// (Run after run, the five outflow stores of a row would read its 18 x-face values in five places of
+// the table: 0.9 us of a 44 us step at 256x128x64 FP16.)  Recorded item by item
 // the table took 0.2 ms at 64x32x8 (free-slip y and z), 4.7 at 1024x512x512, 75 at 65536x2x2; as
 // runs 0.1, 0.1, 0.03.
 struct HaloEdgeRun {
