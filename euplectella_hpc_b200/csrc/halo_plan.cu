@@ -179,18 +179,23 @@ HaloEdges build_halo_edges(const Geo& g, const int bc[6], bool one_by_one) {
 
 cudaError_t put_halo_edges(const HaloEdges& edges, HaloEdgesDevice* out, cudaStream_t st) {
     const int64_t total = edges.first[kHaloBlocks];
-    char* mem = nullptr;
-    cudaError_t e = cudaMalloc(&mem, sizeof(HaloEdge) * total + sizeof(HaloEdgeRun) * edges.runs.size() + 1);
+    HaloEdge* table = nullptr;
+    cudaError_t e = cudaMalloc(&table, sizeof(HaloEdge) * (total + 1));
     if (e != cudaSuccess) return e;
-    out->e = reinterpret_cast<HaloEdge*>(mem);  // the runs behind the table
+    out->e = table;
     for (int b = 0; b <= kHaloBlocks; ++b) out->first[b] = edges.first[b];
     if (total == 0) return cudaSuccess;
-    HaloEdgeRun* runs = reinterpret_cast<HaloEdgeRun*>(mem + sizeof(HaloEdge) * total);
-    e = cudaMemcpyAsync(runs, edges.runs.data(), sizeof(HaloEdgeRun) * edges.runs.size(), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-    k_fill_edges<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(runs, (int)edges.runs.size(), total,
-                                                                  reinterpret_cast<HaloEdge*>(mem));
-    return cudaGetLastError();
+    HaloEdgeRun* runs = nullptr;
+    const size_t bytes = sizeof(HaloEdgeRun) * edges.runs.size();
+    if ((e = cudaMalloc(&runs, bytes)) != cudaSuccess) return e;
+    e = cudaMemcpyAsync(runs, edges.runs.data(), bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) {
+        k_fill_edges<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(runs, (int)edges.runs.size(), total, table);
+        e = cudaGetLastError();
+    }
+    const cudaError_t es = cudaStreamSynchronize(st);
+    cudaFree(runs);
+    return e == cudaSuccess ? es : e;
 }
 
 HaloFace record_halo_face(const Geo& g, const int bc[6], int b) {

@@ -168,7 +168,7 @@ struct HaloEdgesDevice {
     int64_t first[9] = {};
 };
 HaloEdges build_halo_edges(const Geo& g, const int bc[6], bool one_by_one = false);
-// Allocates out->e (cudaFree) and fills it, on st.
+// Allocates out->e (cudaFree) and fills it; synchronises st.
 cudaError_t put_halo_edges(const HaloEdges& edges, HaloEdgesDevice* out, cudaStream_t st);
 
 // One face of the halo away from the edge lines: nodes (a, b) of the face, a = 0 .. na-1 and
